@@ -411,26 +411,24 @@ def true_res(Ah, B, X):
 
 
 # template instance of each recorded sweep form in the mixed (FP32, NV=16) step
-GS_FORM_KERNEL = {"gs_grid": "k_gs3<float,16,0,0,0> (cooperative grid)",
-                  "gs_tile": "k_gs3<float,16,1,1,0,NT> (hybrid blocks, one CTA of NT = 128 or 256 threads each, "
-                             "x tile)",
-                  "gs_window": "k_gs3<float,16,1,0,1,NT> (hybrid blocks, one CTA of NT = 128 or 256 threads each, "
-                               "slot window)",
-                  "gs_gather": "k_gs3<float,16,1,0,0,NT> (hybrid blocks, one CTA of NT = 128 or 256 threads each, "
-                               "per-level gather)",
+GS_FORM_KERNEL = {"gs_grid": "k_gs_flow<float,16> (one sweep on the whole device) or k_gs_block<float,16,XS,512> "
+                             "(one CTA, both sweeps)",
+                  "gs_tile": "k_gs_block<float,16,1,NT> (hybrid blocks, one CTA of NT = 128, 256 or 512 threads each, "
+                             "both sweeps, x tile in shared memory)",
+                  "gs_window": "k_gs_block<float,16,0,NT> (hybrid blocks, one CTA of NT = 128, 256 or 512 threads "
+                               "each, both sweeps, x through the L1)",
                   "gsw_tile": "k_gsw<float,16,1> (hybrid blocks, one warp each, x tile)",
                   "gsw_window": "k_gsw<float,16,2> (hybrid blocks, one warp each, slot window)",
                   "gsw_gather": "k_gsw<float,16,0> (hybrid blocks, one warp each, per-level gather)"}
-# DRAM bytes (read + write) per algorithmic byte of the slot-window sweep,
-# measured by ncu on the 27-point 96^3 case (one launch, 444 blocks, FP32,
-# 128-thread CTAs: the benchmark's configuration)
-GS_TRAFFIC_RATIO = {"gs_window": 1.063}
+# DRAM bytes (read + write) per algorithmic byte of a sweep form, from an ncu
+# capture of the form that runs (none taken of the current kernels yet)
+GS_TRAFFIC_RATIO = {}
 
 
 def gs_roofline(rec, solve_ms, rows):
     """Roofline of the dominant kernel of the mixed step: the hybrid
-    Gauss-Seidel sweep kernel on the finest level (one launch per sweep
-    direction), achieved = algorithmic bytes per launch / CUDA-event time per
+    Gauss-Seidel kernel on the finest level (one launch for both sweeps),
+    achieved = algorithmic bytes per launch / CUDA-event time per
     launch."""
     peak, src = peak_hbm()
     kind = lambda r: "gs" if r["kernel"].startswith("gs") else r["kernel"]
@@ -439,7 +437,7 @@ def gs_roofline(rec, solve_ms, rows):
     if not fine:
         return None
     f = fine[0]
-    name = GS_FORM_KERNEL.get(f["kernel"], "k_gs3") + " (finest level)"
+    name = GS_FORM_KERNEL.get(f["kernel"], "k_gs_block") + " (finest level)"
     per_ms = f["ms"] / f["launches"]
     per_b = f["bytes"] / f["launches"]
     ach = per_b / (per_ms * 1e-3) / 1e9
@@ -813,9 +811,8 @@ def kernel_case(args):
     """One hot kernel alone on a grid of side --n (for profiler captures):
     spmv = the NV=16 product in precision --prec and mode --mode (variant
     --variant; 108 = run kernel); gs = one Gauss-Seidel call (forward and
-    backward sweep) in precision --prec, sequential order (--blocks 0, one
-    cooperative level-ordered launch per sweep) or --blocks hybrid blocks
-    (one CTA per block, one launch per sweep direction)."""
+    backward sweep) in precision --prec, sequential order (--blocks 0) or
+    --blocks hybrid blocks (one CTA per block, both sweeps in one launch)."""
     import ctypes as C
     import torch
     import xamg

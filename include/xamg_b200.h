@@ -35,13 +35,15 @@ long long XAMG_b200_kernel_launches(void);
  * default, it adds two event records per timed launch): on = 1 starts
  * recording every Gauss-Seidel sweep and sparse product (class 1) with its
  * algorithmic bytes, on = 0 stops and discards; returns the previous state.
- * Sweep classes: 2 cooperative grid; hybrid blocks, one CTA per block:
- * 3 x tile in shared memory, 4 slot window, 5 x gathered per level; the same
- * with one warp per block: 6, 7, 8; 0 any other sweep path. */
+ * Sweep classes: 2 single-process order (the whole device, or one CTA for a
+ * narrow schedule); hybrid blocks, one CTA per block: 3 x tile in shared
+ * memory, 4 x read through the L1 (a launch of these runs both sweeps); one
+ * warp per block: 6 x tile, 7 slot window, 8 x gathered per level; 0 any
+ * other sweep path. */
 int XAMG_b200_kernel_timing(int on);
 /* Kernel of the hybrid Gauss-Seidel sweeps in this process: 1 one warp per
- * block, 0 one 256-thread CTA per block (XAMG_GS_SWEEP=warp|cta, read once;
- * both give identical results). */
+ * block, 0 one CTA per block (XAMG_GS_SWEEP=warp|cta, read once; both give
+ * identical results). */
 int XAMG_b200_gs_sweep_kernel(void);
 /* Waits for the device, then writes per (class, operator rows) the launch
  * count, total milliseconds and total algorithmic bytes of the records so far
@@ -243,14 +245,14 @@ int xamg_spmv_set_run_form(int form);
 /* Gauss-Seidel plan (wavefront schedule) for blas2::SGS / csr_SGS
  * (blas2.h:184-281, csr_gs.inl:32-134).  rp/ci are HOST arrays.  block_rows
  * = 0 gives the single-process sweep; > 0 the hybrid block semantics.
- * schedule: 0 = one launch per wavefront level; 1 = automatic (one
- * cooperative launch per sweep with a bounded grid barrier per level, or one
- * CTA per block for hybrid plans); 2 = cooperative grid sweep always. */
+ * schedule: 0 = one launch per wavefront level; 1 = automatic (both sweeps of
+ * a hybrid plan in one launch with one CTA per block, else one launch per sweep
+ * on the whole device or one CTA for a narrow schedule); 2 = the latter always. */
 void *xamg_gs_plan_create(int64_t n, const int *rp_host, const int *ci_host,
                           int64_t block_rows, int schedule);
 /* Give the plan the matrix values (HOST array, CSR order of rp/ci): sweeps in
  * precision prec then run over the plan's level-ordered copy of the matrix
- * with TMA-staged entries (schedules 1 and 2); the val argument of xamg_hsgs
+ * (schedules 1 and 2); the val argument of xamg_hsgs
  * is still used for the hybrid right-hand side. */
 int xamg_gs_plan_set_values(void *plan, const double *val_host, int prec);
 int xamg_gs_plan_levels(void *plan, int *nlev /* [2] */, int *lf, int *lb);
@@ -262,8 +264,7 @@ int xamg_gs_plan_levels(void *plan, int *nlev /* [2] */, int *lf, int *lb);
  * usable afterwards. */
 int XAMG_b200_wait_selftest(int which, int ncta, double limit_s);
 /* Slots of the shared-memory x window of each sweep direction of a hybrid
- * plan with values (0: no window; the window is used when slots * nv * the
- * value size <= 64 KB and the block's x tile does not fit in shared memory). */
+ * plan with values, as the warp-per-block kernel would use it (0: no window). */
 int xamg_gs_plan_slots(void *plan, int *nslots /* [2] */);
 int xamg_gs_plan_error(void *plan);
 void xamg_gs_plan_destroy(void *plan);

@@ -840,7 +840,7 @@ int xamg_gs_plan_set_values(void *plan, const double *val_host, int prec) {
         XCHECK(plan, "null plan");
         PlanHandle *h = (PlanHandle *)plan;
         h->pattern.v.assign(val_host, val_host + h->pattern.nnz());
-        h->plan.build_lcsr(h->pattern, (Prec)prec);
+        h->plan.build_lcsr(h->pattern, (Prec)prec, 0);
     });
 }
 int xamg_gs_plan_levels(void *plan, int *nlev, int *lf, int *lb) {
@@ -857,13 +857,14 @@ int xamg_gs_plan_slots(void *plan, int *nslots) {
     return guard([&] {
         XCHECK(plan, "null plan");
         GsPlan &g = ((PlanHandle *)plan)->plan;
+        g.build_warp(((PlanHandle *)plan)->pattern);
         nslots[0] = g.has_lcsr ? g.lc[0].nslots : 0;
         nslots[1] = g.has_lcsr ? g.lc[1].nslots : 0;
     });
 }
 int XAMG_b200_wait_selftest(int which, int ncta, double limit_s) {
     return guard([&] {
-        XCHECK(which == 0 || which == 1, "which must be 0 (grid barrier) or 1 (mbarrier)");
+        XCHECK(which == 0 || which == 1, "which must be 0 (unwritten element) or 1 (mbarrier)");
         XCHECK(ncta >= 2 && ncta <= 64, "ncta must be 2..64");
         XCHECK(limit_s > 0.0 && limit_s <= 2.0, "limit must be in (0, 2] seconds");
         cudaStream_t s = ctx().stream;
@@ -873,7 +874,7 @@ int XAMG_b200_wait_selftest(int which, int ncta, double limit_s) {
         XCUDA(cudaStreamSynchronize(s));
         int h = 0;
         XCUDA(cudaMemcpy(&h, err.p, sizeof(int), cudaMemcpyDeviceToHost));
-        if (h) throw Error(std::string(which == 0 ? "grid barrier" : "mbarrier") +
+        if (h) throw Error(std::string(which == 0 ? "unwritten element" : "mbarrier") +
                                ": bounded wait expired on the device (error word " + std::to_string(h) + ")",
                            3);
     });
@@ -895,8 +896,7 @@ int xamg_hsgs(void *plan, int prec, int nv, const int *rp, const int *ci, const 
             xk::offblock_resid((Prec)prec, nv, g.n, rp, ci, val, b, x, t, g.brows, s);
             tp = t;
         }
-        g.sweep((Prec)prec, nv, rp, ci, val, invd, tp, x, relax, true, s);
-        g.sweep((Prec)prec, nv, rp, ci, val, invd, tp, x, relax, false, s);
+        g.sweeps((Prec)prec, nv, rp, ci, val, invd, tp, x, relax, s);
         XCUDA(cudaGetLastError());
     });
 }

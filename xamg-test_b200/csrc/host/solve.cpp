@@ -66,6 +66,10 @@ KTimeScope::~KTimeScope() {
     if (on && slot >= 0) cudaEventRecord(g_krecs[slot].e1, s);
 }
 
+void KTimeScope::reclass(KClass k) {
+    if (on && slot >= 0) g_krecs[slot].kclass = (int)k;
+}
+
 int ktime_enable(int on) {
     int old = g_ktime;
     if (!on) kclear();
@@ -177,33 +181,34 @@ static void make_invd(const HostCsr &A, bool f64, bool f32, DBuf &d64, DBuf &d32
 // resolved in the sequential order.  The backward schedule mirrors it.
 void gs_levels_host(const HostCsr &A, i64 brows, std::vector<int> &lf, std::vector<int> &lb) {
     i64 n = A.n;
-    auto inblk = [&](i64 i, i64 c) { return brows <= 0 || (c / brows) == (i / brows); };
     lf.assign(n, 0);
     lb.assign(n, 0);
     std::vector<int> pend(n, 0);
     for (i64 i = 0; i < n; ++i) {
+        const i64 lo = brows > 0 ? i / brows * brows : 0, hi = brows > 0 ? lo + brows : n;
         int L = pend[i];
         for (int j = A.rp[i]; j < A.rp[i + 1]; ++j) {
             i64 c = A.ci[j];
-            if (c < i && inblk(i, c)) L = std::max(L, lf[c] + 1);
+            if (c < i && c >= lo) L = std::max(L, lf[c] + 1);
         }
         lf[i] = L;
         for (int j = A.rp[i]; j < A.rp[i + 1]; ++j) {
             i64 c = A.ci[j];
-            if (c > i && inblk(i, c)) pend[c] = std::max(pend[c], L + 1);
+            if (c > i && c < hi) pend[c] = std::max(pend[c], L + 1);
         }
     }
     std::fill(pend.begin(), pend.end(), 0);
     for (i64 i = n - 1; i >= 0; --i) {
+        const i64 lo = brows > 0 ? i / brows * brows : 0, hi = brows > 0 ? lo + brows : n;
         int L = pend[i];
         for (int j = A.rp[i]; j < A.rp[i + 1]; ++j) {
             i64 c = A.ci[j];
-            if (c > i && inblk(i, c)) L = std::max(L, lb[c] + 1);
+            if (c > i && c < hi) L = std::max(L, lb[c] + 1);
         }
         lb[i] = L;
         for (int j = A.rp[i]; j < A.rp[i + 1]; ++j) {
             i64 c = A.ci[j];
-            if (c < i && inblk(i, c)) pend[c] = std::max(pend[c], L + 1);
+            if (c < i && c >= lo) pend[c] = std::max(pend[c], L + 1);
         }
     }
 }
@@ -311,6 +316,7 @@ void GsPlan::build_offblock(const HostCsr &A, Prec p) {
 // kMaxSlots slots at once.
 constexpr int kSlotAhead = xk::kGsSlotAhead;
 constexpr int kMaxSlots = 4096;
+
 
 void GsPlan::build_slots(int d, const std::vector<int> &order, const std::vector<int> &groups,
                          const std::vector<int> &blev, const std::vector<int> &lrp, const std::vector<int> &lci) {
@@ -432,121 +438,183 @@ void GsPlan::build_slots(int d, const std::vector<int> &order, const std::vector
     for (int g = 0; g < ngroups; ++g) L.nlmax = std::max(L.nlmax, ldd[2 * (size_t)g + 1] - ldd[2 * (size_t)g]);
 }
 
-// Point-to-point waits of the cooperative (GRID) sweep.  Instead of a grid
-// barrier after every level, CTA b publishes the number of levels it has
-// finished, and before level l it waits only for the CTAs that own rows its
-// level-l rows depend on: every row c of the symmetrised pattern of row j
-// (j's own entries and the rows that read j) with a lower level.  Those are
-// the values j reads after their update (c < j) and the rows that must have
-// read j's old value before j changes it (rows c whose entries include j).
-// Per (level, CTA) the list holds each other owner once with the most
-// levels it must have finished.
-void GsPlan::build_grid_deps(int d, const HostCsr &A, const std::vector<int> &lev, const std::vector<int> &order,
-                             const std::vector<int> &desc, int G) {
-    Lcsr &L = lc[d];
-    const int ngroups = (int)(desc.size() / 4 / G);
-    std::vector<int> own(n, -1);
-    for (int l = 0; l < ngroups; ++l)
-        for (int b = 0; b < G; ++b) {
-            const int *dd = &desc[((size_t)l * G + b) * 4];
-            for (int r = dd[0]; r < dd[1]; ++r)
-                if (order[r] >= 0) own[order[r]] = b;
-        }
-    // transpose pattern: the rows whose entries include j
-    std::vector<int> trp(n + 1, 0), tci(A.nnz());
-    for (i64 q = 0; q < A.nnz(); ++q) trp[A.ci[q] + 1]++;
-    for (i64 i = 0; i < n; ++i) trp[i + 1] += trp[i];
-    {
-        std::vector<int> at(trp.begin(), trp.end() - 1);
-        for (i64 i = 0; i < n; ++i)
-            for (int q = A.rp[i]; q < A.rp[i + 1]; ++q) tci[at[A.ci[q]]++] = (int)i;
-    }
-    std::vector<int> dptr((size_t)ngroups * G + 1, 0), deps;
-    std::vector<int> need(G, 0), touched;
-    for (int l = 0; l < ngroups; ++l)
-        for (int b = 0; b < G; ++b) {
-            const int *dd = &desc[((size_t)l * G + b) * 4];
-            touched.clear();
-            auto dep = [&](int c, int lj) {
-                if (c < 0 || c >= n || lev[c] >= lj) return;
-                const int o = own[c];
-                if (o == b || o < 0) return;
-                if (need[o] == 0) touched.push_back(o);
-                need[o] = std::max(need[o], lev[c] + 1);
-            };
-            for (int r = dd[0]; r < dd[1]; ++r) {
-                const int j = order[r];
-                if (j < 0) continue;
-                for (int q = A.rp[j]; q < A.rp[j + 1]; ++q) dep(A.ci[q], lev[j]);
-                for (int q = trp[j]; q < trp[j + 1]; ++q) dep(tci[q], lev[j]);
-            }
-            std::sort(touched.begin(), touched.end());
-            for (int o : touched) {
-                deps.push_back(o);
-                deps.push_back(need[o]);
-                need[o] = 0;
-            }
-            dptr[(size_t)l * G + b + 1] = (int)(deps.size() / 2);
-        }
-    if (deps.empty()) deps.assign(2, 0);
-    upload_ints(L.dptr, dptr);
-    upload_ints(L.deps, deps);
-    L.has_deps = true;
-    if (prog.bytes < (size_t)G * 32) {
-        prog.alloc((size_t)G * 32);
-        XCUDA(cudaMemset(prog.p, 0, prog.bytes));
+static void upload_values(DBuf &dst, const std::vector<double> &v, Prec p) {
+    if (p == Prec::F64) {
+        dst.alloc(sizeof(double) * v.size());
+        XCUDA(cudaMemcpy(dst.p, v.data(), sizeof(double) * v.size(), cudaMemcpyHostToDevice));
+    } else {
+        std::vector<float> f(v.begin(), v.end());
+        dst.alloc(sizeof(float) * f.size());
+        XCUDA(cudaMemcpy(dst.p, f.data(), sizeof(float) * f.size(), cudaMemcpyHostToDevice));
     }
 }
 
-void GsPlan::build_lcsr(const HostCsr &A, Prec p) {
-    if (mode == GsMode::LEVELS) return;
-    lprec = p;
-    int G = 0;
-    if (mode == GsMode::GRID) {
-        int dev = 0;
-        XCUDA(cudaGetDevice(&dev));
-        XCUDA(cudaDeviceGetAttribute(&G, cudaDevAttrMultiProcessorCount, dev));
-        if (G <= 0) G = 148;
+// Cut the level-ordered rows of one direction into items of at most `rows` rows
+// of one level and gs_item_entries entries (a longer row alone); see xk::GsDir
+// for the layout.  The rows of a level are independent, so they are taken
+// longest first: an item's rows then have about the same length.
+void GsPlan::build_items(int d, int rows, const HostCsr &A, Prec p, const std::vector<double> &dinv,
+                         const std::vector<int> &lev, const std::vector<int> &order, const std::vector<int> &groups,
+                         const std::vector<int> &blev) {
+    Lcsr &L = lc[d];
+    const int cap = xk::gs_item_entries(), nb = (int)blev.size() - 1;
+    const int per = p == Prec::F64 ? 2 : 4;  // values in 16 bytes
+    const int pad = (int)(mode == GsMode::BLOCKS ? brows : n);
+    std::vector<int> lo(n, 0), cnt_in(n, 0);  // first row of the row's block, entries inside it
+#pragma omp parallel for schedule(static)
+    for (i64 i = 0; i < n; ++i) {
+        lo[i] = brows > 0 ? (int)(i / brows * brows) : 0;
+        const i64 hi = brows > 0 ? lo[i] + brows : n;
+        int k = 0;
+        for (int j = A.rp[i]; j < A.rp[i + 1]; ++j) k += A.ci[j] >= lo[i] && A.ci[j] < hi;
+        cnt_in[i] = k;
     }
-    std::vector<double> dinv(n, 0.0);
-    for (i64 i = 0; i < n; ++i)
+    std::vector<int> items, bitem(1, 0), imax(std::max(nb, 1), 1), meta, sci;
+    std::vector<double> sva, sinvd;
+    meta.reserve(4 * (size_t)n);
+    sinvd.reserve(n);
+    sci.reserve(A.nnz() + A.nnz() / 4);
+    sva.reserve(A.nnz() + A.nnz() / 4);
+    L.rows = rows;
+    L.ientries = 0;
+    std::vector<std::pair<int, int>> lr;  // (-groups, row) of one level
+    std::vector<int> col;
+    std::vector<double> val;
+    for (int b = 0; b < nb; ++b) {
+        std::vector<int> lastitem;  // last item and items of every level
+        std::vector<int> cnt;
+        for (int g = blev[b]; g < blev[b + 1]; ++g) {
+            const int lz = g - blev[b];
+            lr.clear();
+            for (int r = groups[g]; r < groups[g + 1]; ++r) {
+                const int i = order[r];
+                if (i < 0) continue;
+                lr.push_back({-((cnt_in[i] + 3) / 4), i});
+            }
+            auto shorter = [](const std::pair<int, int> &x, const std::pair<int, int> &y) { return x.first < y.first; };
+            if (!std::is_sorted(lr.begin(), lr.end(), shorter)) std::stable_sort(lr.begin(), lr.end(), shorter);
+            int made = 0;
+            for (size_t s = 0; s < lr.size();) {
+                const int ng = -lr[s].first;
+                size_t z = s + 1;
+                while (z < lr.size() && (int)(z - s) < rows && 4 * ng * (int)(z - s + 1) <= cap) ++z;
+                const int R = (int)(z - s), ne = 4 * ng * R;
+                const int e0 = (int)sci.size(), r0 = (int)(meta.size() / 4);
+                XCHECK((i64)sci.size() + ne < (1ll << 31) - 8, "level-ordered matrix too large");
+                XCHECK(ng < 65536, "row too long for the level-ordered copy");
+                sci.resize(sci.size() + ne, pad);
+                sva.resize(sva.size() + ne, 0.0);
+                int k0 = ng;
+                for (int q = 0; q < R; ++q) {
+                    const int i = lr[s + q].second;
+                    const int c0 = lo[i], first = mode == GsMode::BLOCKS ? c0 : 0;
+                    const i64 c1 = brows > 0 ? c0 + brows : n;
+                    int k = 0;
+                    for (int j = A.rp[i]; j < A.rp[i + 1]; ++j) {
+                        const int c = A.ci[j];
+                        if (c < c0 || c >= c1) continue;
+                        const int gr = k / 4, w = k % 4;
+                        sci[e0 + ((size_t)gr * R + q) * 4 + w] = c - first;
+                        sva[e0 + (size_t)gr * 4 * R + (w / per * R + q) * per + w % per] = A.v[j];
+                        if (lev[c] == lz - 1) k0 = std::min(k0, gr);
+                        ++k;
+                    }
+                    const float f = (float)dinv[i];
+                    int fb;
+                    std::memcpy(&fb, &f, sizeof f);
+                    const int mt[4] = {i, e0, 0, fb};
+                    meta.insert(meta.end(), mt, mt + 4);
+                    sinvd.push_back(dinv[i]);
+                }
+                const int v[4] = {r0, lz, 0, R | std::min(k0, 255) << 8 | ng << 16};
+                items.insert(items.end(), v, v + 4);
+                L.ientries = std::max(L.ientries, ne);
+                ++made;
+                s = z;
+            }
+            imax[b] = std::max(imax[b], made);
+            cnt.push_back(made);
+            lastitem.push_back((int)(items.size() / 4) - 1);
+        }
+        for (size_t k = 0; k < cnt.size(); ++k)
+            if (cnt[k] > 0) items[4 * (size_t)lastitem[k] + 2] = imax[b] - cnt[k];
+        bitem.push_back((int)(items.size() / 4));
+    }
+    L.count = (int)(items.size() / 4);
+    if (items.empty()) items.assign(4, 0);
+    if (meta.empty()) meta.assign(4, 0), sinvd.assign(1, 0.0);
+    if (sci.empty()) sci.assign(8, pad), sva.assign(8, 0.0);
+    upload_ints(L.items, items);
+    upload_ints(L.bitem, bitem);
+    upload_ints(L.imax, imax);
+    upload_ints(L.smeta, meta);
+    upload_ints(L.scb, sci);
+    upload_values(L.sva, sva, p);
+    upload_values(L.sinvd, sinvd, p);
+}
+
+xk::GsDir GsPlan::dir(int d) const {
+    const Lcsr &L = lc[d];
+    return {L.items.as<int4>(), L.bitem.as<int>(), L.imax.as<int>(), L.scb.as<int>(), L.smeta.as<int4>(),
+            L.sva.p, L.sinvd.p, L.rows};
+}
+
+static std::vector<double> inverse_diagonal(const HostCsr &A, Prec p) {
+    std::vector<double> dinv(A.n, 0.0);
+    for (i64 i = 0; i < A.n; ++i)
         for (int j = A.rp[i]; j < A.rp[i + 1]; ++j)
             if (A.ci[j] == i) dinv[i] = p == Prec::F64 ? 1.0 / A.v[j] : (double)(float)(1.0 / (double)(float)A.v[j]);
-    auto inblk = [&](i64 i, i64 c) { return brows <= 0 || (c / brows) == (i / brows); };
-    nnz_in = 0;
-    for (i64 i = 0; i < n; ++i)
-        for (int j = A.rp[i]; j < A.rp[i + 1]; ++j) nnz_in += inblk(i, A.ci[j]);
-    for (int d = 0; d < 2; ++d) {
-        const std::vector<int> &lev = d == 0 ? lf : lb;
-        std::vector<int> order;        // row id per level-ordered row (-1 = padding)
-        std::vector<int> groups(1, 0); // level-group boundaries in `order`
-        std::vector<int> blev(1, 0);
-        order.reserve(n + n / 2);
-        auto emit = [&](i64 r0, i64 r1) {
-            int nl = 0;
-            for (i64 i = r0; i < r1; ++i) nl = std::max(nl, lev[i] + 1);
-            std::vector<int> cnt(nl + 1, 0);
-            for (i64 i = r0; i < r1; ++i) cnt[lev[i] + 1]++;
-            for (int l = 0; l < nl; ++l) cnt[l + 1] += cnt[l];
-            std::vector<int> pos(cnt.begin(), cnt.end() - 1), seg(r1 - r0);
-            for (i64 i = r0; i < r1; ++i) seg[pos[lev[i]]++] = (int)i;
-            for (int l = 0; l < nl; ++l) {
-                for (int q = cnt[l]; q < cnt[l + 1]; ++q) order.push_back(seg[q]);
-                while (order.size() % 4) order.push_back(-1);
-                groups.push_back((int)order.size());
-            }
-            return nl;
-        };
-        if (mode == GsMode::BLOCKS) {
-            for (int b = 0; b < nblocks; ++b) {
-                i64 r0 = (i64)b * brows, r1 = std::min<i64>(n, r0 + brows);
-                blev.push_back(blev.back() + emit(r0, r1));
-            }
-        } else {
-            emit(0, n);
+    return dinv;
+}
+
+// Rows of one direction in schedule order ((block,) level, row), every level
+// padded with row -1 to a multiple of 4 rows: `groups` are the levels'
+// boundaries in `order`, block b's are [blev[b], blev[b + 1]).
+void GsPlan::schedule(int d, std::vector<int> &order, std::vector<int> &groups, std::vector<int> &blev) const {
+    const std::vector<int> &lev = d == 0 ? lf : lb;
+    order.clear();
+    groups.assign(1, 0);
+    blev.assign(1, 0);
+    order.reserve(n + n / 2);
+    auto emit = [&](i64 r0, i64 r1) {
+        int nl = 0;
+        for (i64 i = r0; i < r1; ++i) nl = std::max(nl, lev[i] + 1);
+        std::vector<int> cnt(nl + 1, 0);
+        for (i64 i = r0; i < r1; ++i) cnt[lev[i] + 1]++;
+        for (int l = 0; l < nl; ++l) cnt[l + 1] += cnt[l];
+        std::vector<int> pos(cnt.begin(), cnt.end() - 1), seg(r1 - r0);
+        for (i64 i = r0; i < r1; ++i) seg[pos[lev[i]]++] = (int)i;
+        for (int l = 0; l < nl; ++l) {
+            for (int q = cnt[l]; q < cnt[l + 1]; ++q) order.push_back(seg[q]);
+            while (order.size() % 4) order.push_back(-1);
+            groups.push_back((int)order.size());
         }
+        return nl;
+    };
+    if (mode == GsMode::BLOCKS) {
+        for (int b = 0; b < nblocks; ++b) {
+            i64 r0 = (i64)b * brows, r1 = std::min<i64>(n, r0 + brows);
+            blev.push_back(blev.back() + emit(r0, r1));
+        }
+    } else {
+        blev.push_back(emit(0, n));
+    }
+}
+
+// The warp-per-block sweep's copy (gsw.cu) of a BLOCKS plan: rows in schedule
+// order, each row's entries in the block padded to a multiple of 4 with column
+// -1, one descriptor {r0, r1, e0, e1} a level, and the slot window.
+void GsPlan::build_warp(const HostCsr &A) {
+    if (mode != GsMode::BLOCKS || !has_lcsr || lc[0].desc.p) return;
+    const Prec p = lprec;
+    const std::vector<double> dinv = inverse_diagonal(A, p);
+    auto inblk = [&](i64 i, i64 c) { return (c / brows) == (i / brows); };
+    for (int d = 0; d < 2; ++d) {
+        Lcsr &L = lc[d];
+        std::vector<int> order, groups, blev;
+        schedule(d, order, groups, blev);
         const i64 nr = (i64)order.size();
-        std::vector<int> lrp(nr + 5, 0);
+        std::vector<int> lrp(nr + 5, 0), desc;
         for (i64 r = 0; r < nr; ++r) {
             int i = order[r], k = 0;
             if (i >= 0)
@@ -568,87 +636,58 @@ void GsPlan::build_lcsr(const HostCsr &A, Prec p) {
                     ++q;
                 }
         }
-        // descriptors
-        std::vector<int> desc;
-        const int ngroups = (int)groups.size() - 1;
-        if (mode == GsMode::GRID) {
-            desc.resize((size_t)ngroups * G * 4);
-            // contiguous row ranges of about equal cost (entries + 4 per row),
-            // any row granularity: a level of a few long rows spreads over as
-            // many CTAs as it has rows
-            for (int l = 0; l < ngroups; ++l) {
-                const int a = groups[l], z = groups[l + 1];
-                auto cost = [&](int r) { return (i64)(lrp[r] - lrp[a]) + 4 * (i64)(r - a); };
-                const i64 tot = cost(z);
-                int r = a;
-                for (int b = 0; b < G; ++b) {
-                    const int r0 = r;
-                    if (b == G - 1) {
-                        r = z;
-                    } else {
-                        const i64 goal = tot * (b + 1) / G;
-                        while (r < z && cost(r + 1) <= goal) ++r;
-                    }
-                    int *dd = &desc[((size_t)l * G + b) * 4];
-                    dd[0] = r0; dd[1] = r; dd[2] = lrp[r0]; dd[3] = lrp[r];
-                }
-            }
-        } else {
-            desc.resize((size_t)std::max(ngroups, 1) * 4);
-            for (int l = 0; l < ngroups; ++l) {
-                int *dd = &desc[(size_t)l * 4];
-                dd[0] = groups[l]; dd[1] = groups[l + 1]; dd[2] = lrp[groups[l]]; dd[3] = lrp[groups[l + 1]];
-            }
+        desc.resize((size_t)std::max(L.nlev, 1) * 4);
+        L.emax = L.rmax = L.lmax = 0;
+        for (int l = 0; l < L.nlev; ++l) {
+            int *dd = &desc[(size_t)l * 4];
+            dd[0] = groups[l]; dd[1] = groups[l + 1]; dd[2] = lrp[groups[l]]; dd[3] = lrp[groups[l + 1]];
+            L.emax = std::max(L.emax, dd[3] - dd[2]);
+            L.rmax = std::max(L.rmax, ((dd[1] + 3) & ~3) - (dd[0] & ~3));
         }
+        for (size_t b = 0; b + 1 < blev.size(); ++b) L.lmax = std::max(L.lmax, blev[b + 1] - blev[b]);
         if (order.empty()) order.push_back(-1);
-        Lcsr &L = lc[d];
-        L.nlev = ngroups;
-        L.ncta = mode == GsMode::GRID ? G : nblocks;
-        L.emax = 0;
-        L.rmax = 0;
-        for (size_t q = 0; q + 3 < desc.size(); q += 4) {
-            L.emax = std::max(L.emax, desc[q + 3] - desc[q + 2]);
-            L.rmax = std::max(L.rmax, ((desc[q + 1] + 3) & ~3) - (desc[q] & ~3));
-        }
-        L.lmax = 0;
-        if (mode == GsMode::BLOCKS)
-            for (size_t b = 0; b + 1 < blev.size(); ++b) L.lmax = std::max(L.lmax, blev[b + 1] - blev[b]);
         upload_ints(L.lrp, lrp);
         upload_ints(L.lci, lci);
         upload_ints(L.lrow, order);
         upload_ints(L.desc, desc);
         upload_ints(L.blev, blev);
-        if (mode == GsMode::BLOCKS) build_slots(d, order, groups, blev, lrp, lci);
-        if (mode == GsMode::GRID) build_grid_deps(d, A, lev, order, desc, G);
-        if (p == Prec::F64) {
-            L.lva.alloc(sizeof(double) * lv.size());
-            XCUDA(cudaMemcpy(L.lva.p, lv.data(), sizeof(double) * lv.size(), cudaMemcpyHostToDevice));
-            L.linvd.alloc(sizeof(double) * li.size());
-            XCUDA(cudaMemcpy(L.linvd.p, li.data(), sizeof(double) * li.size(), cudaMemcpyHostToDevice));
-        } else {
-            std::vector<float> f(lv.begin(), lv.end()), g(li.begin(), li.end());
-            L.lva.alloc(sizeof(float) * f.size());
-            XCUDA(cudaMemcpy(L.lva.p, f.data(), sizeof(float) * f.size(), cudaMemcpyHostToDevice));
-            L.linvd.alloc(sizeof(float) * g.size());
-            XCUDA(cudaMemcpy(L.linvd.p, g.data(), sizeof(float) * g.size(), cudaMemcpyHostToDevice));
-        }
+        upload_values(L.lva, lv, p);
+        upload_values(L.linvd, li, p);
+        build_slots(d, order, groups, blev, lrp, lci);
     }
-    has_lcsr = true;
 }
 
-// The slot window can be switched off (XAMG_GS_NO_SLOT_WINDOW set) to run
-// the per-level gather form of the same sweeps, whose results are identical.
-// Likewise the point-to-point waits of the cooperative sweep
-// (XAMG_GS_GRID_BARRIER set: a grid barrier after every level instead).
-static bool grid_deps_on() {
-    static const bool on = std::getenv("XAMG_GS_GRID_BARRIER") == nullptr;
-    return on;
+void GsPlan::build_lcsr(const HostCsr &A, Prec p, int nv) {
+    if (mode == GsMode::LEVELS) return;
+    lprec = p;
+    const std::vector<double> dinv = inverse_diagonal(A, p);
+    nnz_in = 0;
+    for (i64 i = 0; i < n; ++i) {
+        const i64 lo = brows > 0 ? i / brows * brows : 0, hi = brows > 0 ? lo + brows : n;
+        for (int j = A.rp[i]; j < A.rp[i + 1]; ++j) nnz_in += A.ci[j] >= lo && A.ci[j] < hi;
+    }
+    for (int d = 0; d < 2; ++d) {
+        const std::vector<int> &lev = d == 0 ? lf : lb;
+        std::vector<int> order, groups, blev;
+        schedule(d, order, groups, blev);
+        lc[d].nlev = (int)groups.size() - 1;
+        // of unknown width: eight rows, a warp's of 64-byte rows
+        build_items(d, nv == 0 ? 8 : xk::gs_rows_per_item(p, nv), A, p, dinv, lev, order, groups, blev);
+    }
+    if (mode == GsMode::GRID && nv > 0) wmid.alloc((size_t)n * nv * prec_size(p));
+    has_lcsr = true;
+    lc[0].desc.release();  // the warp kernel's copy of earlier values
+    if (gs_warp_sweep()) build_warp(A);
 }
+
+// The slot window of the warp-per-block sweep can be switched off
+// (XAMG_GS_NO_SLOT_WINDOW set) to run its per-level gather form, whose results
+// are identical.
 static bool slot_window_on() {
     static const bool on = std::getenv("XAMG_GS_NO_SLOT_WINDOW") == nullptr;
     return on;
 }
-// Hybrid sweeps: one 256-thread CTA per block, or one warp per block
+// Hybrid sweeps: one CTA per block, or one warp per block
 // (XAMG_GS_SWEEP=warp; XAMG_GS_SWEEP=cta selects the CTA kernel explicitly).
 // Results are identical.
 constexpr bool kWarpSweepDefault = false;
@@ -664,55 +703,87 @@ static bool warp_sweep_on() {
 
 int gs_warp_sweep() { return warp_sweep_on() ? 1 : 0; }
 
-void GsPlan::sweep(Prec p, int nv, const int *rp, const int *ci, const void *val,
-                   const void *invd, const void *t, void *x, const void *relax, bool forward,
-                   cudaStream_t s) {
-    int nl = forward ? nlf : nlb;
-    const std::vector<int> &hl = forward ? hlf : hlb;
-    const int *perm = (forward ? permf : permb).as<int>();
-    if (nl == 0) return;
-    if (has_lcsr && p == lprec && (mode == GsMode::GRID || mode == GsMode::BLOCKS)) {
-        const Lcsr &L = lc[forward ? 0 : 1];
-        unsigned *bar = sync.as<unsigned>();
-        int *err = (int *)(sync.as<char>() + kSyncErrOffset);
-        int md = mode == GsMode::BLOCKS ? 1 : 0;
-        // the block's x tile in shared memory when it fits; a tile that allows
-        // only one CTA per SM only when the blocks fit in one wave anyway
-        // (otherwise the gather form, two CTAs per SM, finishes sooner)
-        const i64 tile = (i64)brows * nv * (i64)prec_size(p);
-        int xs = md == 1 && (tile <= xk::gs_lcsr_xs_bytes_two_per_sm() ||
-                             (tile <= xk::gs_lcsr_max_xs_bytes() && nblocks <= sm_count()));
-        // one sweep: in-block entries (column + value), per row its id, offset
-        // and inverse diagonal, and t read, x read, x written
-        const double sv = (double)prec_size(p);
-        xk::GsSlotWin win{L.lslot.as<int>(), L.ldd.as<int2>(), L.ldpre.as<int2>(), L.ld.as<int2>(), L.nslots};
-        xk::GsDeps gd{nullptr, nullptr, nullptr};
-        if (md == 0 && L.has_deps && grid_deps_on()) gd = {L.dptr.as<int>(), L.deps.as<int2>(), prog.as<unsigned>()};
-        const bool slots = md == 1 && !xs && L.nslots > 0 && slot_window_on() &&
-                           (size_t)L.nslots * nv * prec_size(p) <= (size_t)xk::gs_slot_window_bytes() &&
-                           nv * prec_size(p) >= 16;
-        const double gbytes = (double)nnz_in * (4 + sv) + (double)n * (8 + sv) + 3.0 * n * nv * sv;
-        if (md == 1 && warp_sweep_on()) {
-            const int wslots = L.nslots > 0 && slot_window_on() ? L.nslots : 0;
-            const xk::GswShape z = xk::gsw_shape(prec_size(p), nv, L.ncta, sm_count(), brows, wslots, L.emax,
-                                                 L.rmax, L.lmax, L.nlmax);
-            if (z.xm >= 0) {
-                const KClass kw = z.xm == 1 ? KClass::GSW_TILE : z.xm == 2 ? KClass::GSW_WINDOW : KClass::GSW_GATHER;
-                KTimeScope kt(kw, n, gbytes, s);
-                XCUDA(xk::gs_sweep_warp(p, nv, z, L.ncta, L.desc.as<int>(), L.blev.as<int>(), L.lrp.as<int>(),
-                                        z.xm == 2 ? L.lcs.as<int>() : L.lci.as<int>(), L.lva.p, L.lrow.as<int>(),
-                                        L.linvd.p, t, x, relax, brows, n, z.xm == 2 ? &win : nullptr, L.lmax, s));
+bool GsPlan::sweeps_lcsr(Prec p, int nv, const void *t, void *x, const void *relax, cudaStream_t s) {
+    int *err = (int *)(sync.as<char>() + kSyncErrOffset);
+    const Lcsr &If = lc[0], &Ib = lc[1];
+    // one sweep: in-block entries (column + value), per row its id, offset
+    // and inverse diagonal, and t read, x read, x written
+    const double sv = (double)prec_size(p);
+    const double gbytes = (double)nnz_in * (4 + sv) + (double)n * (8 + sv) + 3.0 * n * nv * sv;
+    const xk::GsDir f = dir(0), b = dir(1);
+    const int emax = std::max(If.ientries, Ib.ientries);
+    if (mode == GsMode::BLOCKS) {
+        bool tile = false;
+        KTimeScope kt(KClass::GS_WINDOW, n, 2 * gbytes, s);
+        XCUDA(xk::gs_sweep_block(p, nv, nblocks, f, b, t, x, relax, brows, n, emax, err, &tile, s));
+        if (tile) kt.reclass(KClass::GS_TILE);
+        return true;
+    }
+    // a narrow schedule runs in one CTA of 16 warps: up to 8 items a level it
+    // is the faster one (FP64, NV = 4, 27-point 32^3 hierarchy, both sweeps of a
+    // level: 370 rows 386 against 726 us, 2087 rows 727 against 884, 8192 rows
+    // 900 against 900, 32768 rows 1492 against 805)
+    if (If.count <= 8 * lc[0].nlev) {
+        bool tile = false;
+        KTimeScope kt(KClass::GS_GRID, n, 2 * gbytes, s);
+        XCUDA(xk::gs_sweep_block(p, nv, 1, f, b, t, x, relax, n, n, emax, err, &tile, s));
+        return true;
+    }
+    const size_t need = (size_t)n * nv * prec_size(p);
+    if (wmid.bytes < need) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        XCUDA(cudaStreamIsCapturing(s, &st));
+        if (st != cudaStreamCaptureStatusNone) return false;
+        wmid.alloc(need);
+    }
+    {
+        KTimeScope kt(KClass::GS_GRID, n, gbytes, s);
+        XCUDA(xk::gs_sweep_flow(p, nv, f, If.count, lc[0].nlev, 1, t, x, wmid.p, relax, n, emax, err, s));
+    }
+    KTimeScope kt(KClass::GS_GRID, n, gbytes, s);
+    XCUDA(xk::gs_sweep_flow(p, nv, b, Ib.count, lc[1].nlev, 0, t, wmid.p, x, relax, n, emax, err, s));
+    return true;
+}
+
+void GsPlan::sweeps(Prec p, int nv, const int *rp, const int *ci, const void *val, const void *invd, const void *t,
+                    void *x, const void *relax, cudaStream_t s) {
+    if (nlf == 0) return;
+    if (has_lcsr && p == lprec && mode != GsMode::LEVELS) {
+        if (mode == GsMode::BLOCKS && gs_warp_sweep() && lc[0].desc.p) {
+            const int wslots[2] = {lc[0].nslots > 0 && slot_window_on() ? lc[0].nslots : 0,
+                                   lc[1].nslots > 0 && slot_window_on() ? lc[1].nslots : 0};
+            xk::GswShape z[2];
+            for (int d = 0; d < 2; ++d)
+                z[d] = xk::gsw_shape(prec_size(p), nv, nblocks, sm_count(), brows, wslots[d], lc[d].emax, lc[d].rmax,
+                                     lc[d].lmax, lc[d].nlmax);
+            if (z[0].xm >= 0 && z[1].xm >= 0) {
+                const double sv = (double)prec_size(p);
+                const double gbytes = (double)nnz_in * (4 + sv) + (double)n * (8 + sv) + 3.0 * n * nv * sv;
+                for (int d = 0; d < 2; ++d) {
+                    const Lcsr &L = lc[d];
+                    const int xm = z[d].xm;
+                    const KClass kw = xm == 1 ? KClass::GSW_TILE : xm == 2 ? KClass::GSW_WINDOW : KClass::GSW_GATHER;
+                    KTimeScope kt(kw, n, gbytes, s);
+                    xk::GsSlotWin win{L.lslot.as<int>(), L.ldd.as<int2>(), L.ldpre.as<int2>(), L.ld.as<int2>(),
+                                      L.nslots};
+                    XCUDA(xk::gs_sweep_warp(p, nv, z[d], nblocks, L.desc.as<int>(), L.blev.as<int>(), L.lrp.as<int>(),
+                                            xm == 2 ? L.lcs.as<int>() : L.lci.as<int>(), L.lva.p, L.lrow.as<int>(),
+                                            L.linvd.p, t, x, relax, brows, n, xm == 2 ? &win : nullptr, L.lmax, s));
+                }
                 return;
             }
         }
-        const KClass kc = md == 0 ? KClass::GS_GRID : xs ? KClass::GS_TILE : slots ? KClass::GS_WINDOW : KClass::GS_GATHER;
-        KTimeScope kt(kc, n, gbytes, s);
-        XCUDA(xk::gs_sweep_lcsr(p, nv, md, xs, L.nlev, L.ncta, L.desc.as<int>(), L.blev.as<int>(),
-                                L.lrp.as<int>(), slots ? L.lcs.as<int>() : L.lci.as<int>(), L.lva.p,
-                                L.lrow.as<int>(), L.linvd.p, t, x, relax, brows, n, bar, err, L.emax,
-                                slots ? &win : nullptr, gd.dptr ? &gd : nullptr, s));
-        return;
+        if (sweeps_lcsr(p, nv, t, x, relax, s)) return;
     }
+    sweep_csr(p, nv, rp, ci, val, invd, t, x, relax, true, s);
+    sweep_csr(p, nv, rp, ci, val, invd, t, x, relax, false, s);
+}
+
+void GsPlan::sweep_csr(Prec p, int nv, const int *rp, const int *ci, const void *val, const void *invd, const void *t,
+                       void *x, const void *relax, bool forward, cudaStream_t s) {
+    int nl = forward ? nlf : nlb;
+    const std::vector<int> &hl = forward ? hlf : hlb;
+    const int *perm = (forward ? permf : permb).as<int>();
     if (mode == GsMode::BLOCKS) {
         if (forward)
             xk::gs_blocks(p, nv, nblocks, bblevf.as<int>(), blptrf.as<int>(), bpermf.as<int>(),
@@ -929,8 +1000,7 @@ struct HSGS : Solver {
             tp = t.p();
         }
         const DCsr &A = *op.A;
-        op.gs->sweep(prec, nv, A.rpp(), A.cip(), A.val(prec), op.invd, tp, x.p(), relax.p, true, s);
-        op.gs->sweep(prec, nv, A.rpp(), A.cip(), A.val(prec), op.invd, tp, x.p(), relax.p, false, s);
+        op.gs->sweeps(prec, nv, A.rpp(), A.cip(), A.val(prec), op.invd, tp, x.p(), relax.p, s);
     }
     bool residual_check(DVec &x, const DVec &b, bool initial) {
         cudaStream_t s = ctx().stream;
@@ -1248,7 +1318,7 @@ struct MultiGrid : Solver {
                 op.gs = &m.gs_pre;
             } else {
                 g.build(hA, br, md);
-                g.build_lcsr(hA, m.prec);
+                g.build_lcsr(hA, m.prec, nv);
                 g.build_offblock(hA, m.prec);
                 op.gs = &g;
             }
@@ -1798,7 +1868,7 @@ static std::unique_ptr<Solver> make_solver(const GlobalParams &gp, const std::st
         if (m == "HSGS") {
             i64 br = hsgs_block_rows(pl, A.h.n);
             o->gs.build(A.h, br, gs_mode_from(pl.has("gs_schedule") ? pl.get_string("gs_schedule") : "auto", br, A.h.n));
-            o->gs.build_lcsr(A.h, prec);
+            o->gs.build_lcsr(A.h, prec, nv);
             o->gs.build_offblock(A.h, prec);
             op.gs = &o->gs;
             auto h = std::unique_ptr<HSGS>(new HSGS());

@@ -81,9 +81,9 @@ struct DCsr {
 // Wavefront schedule of the forward and backward Gauss-Seidel sweeps of one
 // matrix (optionally restricted to hybrid blocks of `brows` rows).
 // Sweep schedules: LEVELS launches one kernel per wavefront level; GRID runs
-// a whole sweep in one cooperative launch with a bounded grid barrier per
-// level; BLOCKS (hybrid plans only) runs each block in its own CTA with CTA
-// barriers, both sweeps in one launch.
+// a whole sweep in one launch (cooperative over the device, or one CTA for a
+// narrow schedule); BLOCKS (hybrid plans only) runs each block in its own CTA,
+// both sweeps in one launch.
 enum class GsMode : int { LEVELS = 0, GRID = 1, BLOCKS = 2 };
 
 // Synchronisation words of a plan's sweeps, each group on its own 128-byte
@@ -106,9 +106,8 @@ struct GsPlan {
     struct Lcsr {
         DBuf lrp, lci, lva, lrow, linvd, desc, blev;
         int nlev = 0;  // GRID: levels; BLOCKS: unused (per-block counts in blev)
-        int ncta = 0;  // CTAs of the launch the descriptors were built for
-        int emax = 0;  // most entries of one CTA in one level
-        int rmax = 0;  // most rows of one CTA in one level (span rounded out to 4)
+        int emax = 0;  // BLOCKS: most entries of one block in one level
+        int rmax = 0;  // BLOCKS: most rows of one block in one level (span rounded out to 4)
         int lmax = 0;  // BLOCKS: most levels of one block
         int nlmax = 0; // BLOCKS with a slot window: longest load list of one level
         // BLOCKS: slot-mapped x window (see build_slots): column indices
@@ -117,12 +116,13 @@ struct GsPlan {
         // levels ahead of their first use
         DBuf lcs, lslot, ldd, ldpre, ld;
         int nslots = 0;  // 0: no window (too many rows live at once)
-        // GRID: per (level, CTA) the CTAs whose earlier levels this one's rows
-        // depend on, {cta, levels it must have finished} (see build_grid_deps)
-        DBuf dptr, deps;
-        bool has_deps = false;
+        // gs.cu's copy: items of a few rows (see xk::GsDir)
+        DBuf items, bitem, imax, scb, sva, sinvd, smeta;
+        int rows = 0, count = 0, ientries = 0;  // most rows of an item, items, most entries of one
     } lc[2];
-    DBuf prog;  // GRID: per-CTA count of finished levels (32-byte stride)
+    // GRID: the vector between the forward and the backward sweep (the plan's
+    // sweeps run one at a time)
+    DBuf wmid;
     bool has_lcsr = false;
     i64 nnz_in = 0;  // entries inside the rows' blocks (all entries without blocks)
     Prec lprec = Prec::F64;
@@ -132,19 +132,30 @@ struct GsPlan {
     DCsr aoff;
     Prec aprec = Prec::F64;
     void build(const HostCsr &A, i64 brows_, GsMode mode_);
-    // store the level-ordered matrix copies in precision p (values from A)
-    void build_lcsr(const HostCsr &A, Prec p);
+    // store the level-ordered matrix copies in precision p (values from A) for
+    // sweeps of nv columns (0: of any width)
+    void build_lcsr(const HostCsr &A, Prec p, int nv);
     void build_offblock(const HostCsr &A, Prec p);
-    // point-to-point dependencies of one sweep direction of a GRID plan
-    void build_grid_deps(int d, const HostCsr &A, const std::vector<int> &lev, const std::vector<int> &order,
-                         const std::vector<int> &desc, int G);
+    // gs.cu's copy of one sweep direction (called by build_lcsr)
+    void build_items(int d, int rows, const HostCsr &A, Prec p, const std::vector<double> &dinv,
+                     const std::vector<int> &lev, const std::vector<int> &order, const std::vector<int> &groups,
+                     const std::vector<int> &blev);
+    xk::GsDir dir(int d) const;
+    void schedule(int d, std::vector<int> &order, std::vector<int> &groups, std::vector<int> &blev) const;
+    // the warp-per-block kernel's copy of the values of build_lcsr (same A)
+    void build_warp(const HostCsr &A);
     // slot window of one sweep direction of a BLOCKS plan (called by build_lcsr)
     void build_slots(int d, const std::vector<int> &order, const std::vector<int> &groups,
                      const std::vector<int> &blev, const std::vector<int> &lrp, const std::vector<int> &lci);
-    // forward (or backward) sweep; in BLOCKS mode the forward call runs both
-    // sweeps and the backward call does nothing
-    void sweep(Prec p, int nv, const int *rp, const int *ci, const void *val, const void *invd,
-               const void *t, void *x, const void *relax, bool forward, cudaStream_t s);
+    // forward and backward sweep
+    void sweeps(Prec p, int nv, const int *rp, const int *ci, const void *val, const void *invd, const void *t,
+                void *x, const void *relax, cudaStream_t s);
+    // over the level-ordered copy by CTAs; false: not possible now (no vector
+    // between the sweeps and none may be allocated during a stream capture)
+    bool sweeps_lcsr(Prec p, int nv, const void *t, void *x, const void *relax, cudaStream_t s);
+    // one direction by the kernels that need no level-ordered copy
+    void sweep_csr(Prec p, int nv, const int *rp, const int *ci, const void *val, const void *invd, const void *t,
+                   void *x, const void *relax, bool forward, cudaStream_t s);
     int error_flag() const;
 };
 GsMode gs_mode_from(const std::string &s, i64 brows, i64 n);

@@ -85,48 +85,58 @@ void gs_blocks(Prec p, int nv, int nblocks, const int *blevf, const int *lptrf, 
                const void *val, const void *invd, const void *t, void *x, const void *relax,
                i64 brows, cudaStream_t s);
 
-// Sweep over a level-ordered copy of the matrix (gs.cu).  mode 0: ncta CTAs
-// share every level with a bounded grid barrier (cooperative launch); mode 1:
-// CTA b owns hybrid block b (ncta blocks).  desc holds one int4 {r0, r1, e0,
-// e1} per (level, CTA): mode 0 at [l*ncta + b], mode 1 at [blev[b] + l].
-// lrow/invd are in level order (lrow = -1 marks padding rows).  xs = 1 keeps
-// the block's x tile in shared memory (mode 1, brows*nv*sizeof(T) <=
-// gs_lcsr_max_xs_bytes()).  Mode 0 uses the first 256 bytes of gbar
-// (8-byte aligned) for the grid barrier and zeroes them before the launch;
-// err must lie outside them.  emax: the most entries any CTA processes in one
-// level (sizes the shared-memory gather buffer; <= 0 = unknown).
-//
-// Slot window of a BLOCKS sweep whose x tile does not fit (win may be null):
+// Sweeps over a level-ordered copy of the matrix (gs.cu).  GsDir: one sweep
+// direction, its rows cut into items of at most `rows` rows of one level.  The
+// rows of an item are padded to the same number of groups of four entries
+// (column: one past a full block, value +0); its entries are stored from e0 on in
+// CSR order by group, then in pieces of 16 bytes by (piece of the group, row):
+// columns (lci, counted from the block's first row) and values (lva) each.
+// items: {first row, level, extra, packed} with packed = rows | k0 << 8 | groups
+// << 16 and extra = the items that the block's widest level has more than this
+// one (on the level's last item, else 0).  k0: the groups ahead of the first one
+// in which a row of the item reads the previous level.  imax[b]: items of the
+// widest level of block b.  meta:
+// per level-ordered row {row id, e0 of its item, 0, FP32 inverse diagonal},
+// linvd: the inverse diagonals in the sweep's precision.  Items of block b:
+// [bitem[b], bitem[b + 1]) in level order.
+struct GsDir {
+    const int4 *items;
+    const int *bitem, *imax, *lci;
+    const int4 *meta;
+    const void *lva, *linvd;
+    int rows;
+};
+// most rows of a warp; entries of an item beyond which its rows are fewer (a
+// single row may have more)
+int gs_rows_per_item(Prec p, int nv);
+int gs_item_entries();
+// Forward and backward sweep of every block in one launch, one CTA per block
+// (512 threads when there is at most one block per SM, else 256).  emax: the
+// most entries of one item.  *tile: whether the x tile was in shared memory.
+// An expired wait sets *err.
+cudaError_t gs_sweep_block(Prec p, int nv, int nblocks, const GsDir &f, const GsDir &b, const void *t, void *x,
+                           const void *relax, i64 brows, i64 n, int emax, int *err, bool *tile, cudaStream_t s);
+// One single-process sweep on the whole device: xin (values before the sweep)
+// to xout, which the call fills with a sentinel first (distinct vectors).
+cudaError_t gs_sweep_flow(Prec p, int nv, const GsDir &d, int nitems, int nlev, int forward, const void *t,
+                          const void *xin, void *xout, const void *relax, i64 n, int emax, int *err, cudaStream_t s);
+
+// Slot window of a warp-per-block sweep whose x tile does not fit (gsw.cu):
 // lci then holds slot numbers instead of columns, lslot gives each
 // level-ordered row's slot, and ld holds {row, slot} pairs: for level group g
 // the range ldd[g] = {first, end} lists the rows first used kGsSlotAhead
 // levels after g, ldpre[b] those first used in block b's first kGsSlotAhead
 // levels (each range starts at an even index and has an even length, padded
-// with {-1, -1}).  Used when nslots * nv * sizeof(T) <= gs_slot_window_bytes()
-// and a row of x is a multiple of 16 bytes; otherwise the level gathers.
+// with {-1, -1}).
 constexpr int kGsSlotAhead = 4;
 struct GsSlotWin {
     const int *lslot;
     const int2 *ldd, *ldpre, *ld;
     int nslots;
 };
-// Point-to-point waits of a GRID sweep (deps may be null: a grid barrier
-// after every level): CTA b publishes at prog[b * 8] the number of levels it
-// has finished; before level l it waits for deps[dptr[l*ncta + b] ..
-// dptr[l*ncta + b + 1]) = {cta, levels that CTA must have finished}.  prog
-// holds ncta * 8 words and is zeroed by the launcher.
-struct GsDeps {
-    const int *dptr;
-    const int2 *deps;
-    unsigned *prog;
-};
-cudaError_t gs_sweep_lcsr(Prec p, int nv, int mode, int xs, int nlev, int ncta, const int *lev_row,
-                          const int *blev, const int *lrp, const int *lci, const void *lva,
-                          const int *lrow, const void *invd, const void *t, void *x,
-                          const void *relax, i64 brows, i64 n, unsigned *gbar, int *err,
-                          int emax, const GsSlotWin *win, const GsDeps *deps, cudaStream_t s);
-// Hybrid sweep with one warp per block (gsw.cu): same arrays and results as
-// gs_sweep_lcsr mode 1.  gsw_shape picks the x form (xm 1 tile, 2 slot
+// Hybrid sweep of one direction with one warp per block (gsw.cu) over the same
+// level-ordered rows, same results; desc holds one int4 {r0, r1, e0, e1} per
+// level at [blev[b] + l].  gsw_shape picks the x form (xm 1 tile, 2 slot
 // window, 0 per-level gather; -1 none fits) and the record stages for the
 // plan's extremes: emax entries, rmax rows (rounded out to 4) and nlmax
 // window loads in one level of one block, lmax levels in one block.
@@ -140,14 +150,11 @@ cudaError_t gs_sweep_warp(Prec p, int nv, const GswShape &z, int nblocks, const 
                           const int *lrp, const int *lci, const void *lva, const int *lrow, const void *invd,
                           const void *t, void *x, const void *relax, i64 brows, i64 n, const GsSlotWin *win,
                           int lmax, cudaStream_t s);
-// Bounded-wait self-test (which 0: grid barrier with one CTA missing; 1:
+// Bounded-wait self-test (which 0: a vector element that no CTA writes; 1: an
 // mbarrier phase that nothing completes), limit in ns; words: 256 bytes of
 // device scratch, err: one device int (0 after a wait that did not run out).
 cudaError_t wait_selftest(int which, int ncta, unsigned long long limit_ns, unsigned *words, int *err,
                           cudaStream_t s);
-int gs_lcsr_max_xs_bytes();
-int gs_lcsr_xs_bytes_two_per_sm();
-int gs_slot_window_bytes();
 
 // Hybrid Gauss-Seidel right-hand side: t = 1*b + (-1)*(sum over the entries
 // outside the row's block of a_ij x_j)   (blas2.h:226-259)
