@@ -29,9 +29,9 @@ int xcnn_conv3d(const void *in, int ics, int ic0, int cin, const void *w, const 
                 void *out, int ocs, int oc0, int cout, int nb, int d, int h, int wd, int flags,
                 void *stream);
 /* Kernel choice of xcnn_conv3d (same convolution either way): 1 (default) =
- * box kernel where the volume tiles into 2 x 8 x 8 voxel boxes (each input
- * voxel staged once per 16-channel chunk), 0 = voxel-tile kernel.  Returns the
- * previous setting. */
+ * box kernel unless padding the volume to boxes of 8 x 8 in (y, x) costs more
+ * than it saves (each input voxel staged once per 16-channel chunk), 0 =
+ * voxel-tile kernel.  Returns the previous setting. */
 int xcnn_set_box_conv(int on);
 /* 1 = xcnn_conv3d runs on the 5th-generation tensor cores (tcgen05.mma with a
  * TMEM accumulator; the same convolution, FP32 accumulation in another order);

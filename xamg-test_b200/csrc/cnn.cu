@@ -15,13 +15,15 @@
 //              epilogue adds the bias, applies ReLU and stores BF16 (or adds
 //              to the stored value, for gradients that meet at a skip).
 //   wgrad    : dW[co][t][ci] += sum_p g[p][co] * in[p + off(t)][ci], one CTA
-//              per (voxel slice, tap, 16-channel chunk of ci), operands loaded
-//              transposed by ldmatrix.trans, FP32 atomics into dW.
+//              per (set of boxes, 16-channel chunk of ci, up to 64 channels of
+//              co) with all 27 taps, operands loaded transposed by
+//              ldmatrix.trans, FP32 atomics into dW.
 //   backward data = conv3d of the gradient with the flipped, transposed
 //              weights (weight_flip).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include "kernels.cuh"
+#include <algorithm>
 #include <cstdint>
 #include <cstdio>
 
@@ -54,10 +56,15 @@ __device__ __forceinline__ void ldm_x2(unsigned (&r)[2], const void *p) {
                  : "=r"(r[0]), "=r"(r[1])
                  : "r"(smem_u32(p)));
 }
-__device__ __forceinline__ void ldm_x4_t(unsigned (&r)[4], const void *p) {
+__device__ __forceinline__ void ldm_x4_a(unsigned (&r)[4], unsigned a) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(a));
+}
+__device__ __forceinline__ void ldm_x4_ta(unsigned (&r)[4], unsigned a) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-                 : "r"(smem_u32(p)));
+                 : "r"(a));
 }
 
 // D = A (16x16, row) * B (16x8, col) + D, BF16 inputs, FP32 accumulate
@@ -75,31 +82,10 @@ __device__ __forceinline__ void mma16816(float (&d)[4], const unsigned (&a)[4], 
 // one ldmatrix hit 8 distinct bank groups.
 __device__ __forceinline__ int sw32(int r, int h) { return r * 32 + ((h ^ ((r >> 2) & 1)) << 4); }
 
-// Rows of nch 16-byte chunks (nch a power of two, >= 2): chunk index XOR a
-// function of the row that spreads 8 consecutive rows over 8 bank groups.
-__device__ __forceinline__ int swn(int r, int ch, int nch) {
-    const int g = nch >= 8 ? 8 : nch;
-    const int per = 8 / g;
-    return r * nch * 16 + ((ch ^ ((r / per) & (g - 1))) << 4);
-}
-
 struct Vol {
     int nb, d, h, w;
     __host__ __device__ __forceinline__ i64 count() const { return (i64)nb * d * h * w; }
 };
-
-// neighbour of linear voxel v at tap t; -1 outside the volume
-__device__ __forceinline__ i64 nbr(const Vol &g, i64 v, int t) {
-    const int x = (int)(v % g.w);
-    const i64 q = v / g.w;
-    const int y = (int)(q % g.h);
-    const i64 q2 = q / g.h;
-    const int z = (int)(q2 % g.d);
-    const int dz = t / 9 - 1, dy = (t / 3) % 3 - 1, dx = t % 3 - 1;
-    const int zz = z + dz, yy = y + dy, xx = x + dx;
-    if (zz < 0 || zz >= g.d || yy < 0 || yy >= g.h || xx < 0 || xx >= g.w) return -1;
-    return v + ((i64)dz * g.h + dy) * g.w + dx;
-}
 
 constexpr int BM = 128;  // voxels per CTA tile
 constexpr int NS = 4;    // pipeline stages
@@ -234,223 +220,394 @@ __global__ void __launch_bounds__(128) k_conv3d(const bf16 *__restrict__ in, int
             }
 }
 
-// conv3d on boxes: the CTA's 128 output voxels form a bz x by x bx box (the
-// volume's sides are multiples of it); for every 16-channel chunk the box's
-// halo ((bz+2)(by+2)(bx+2) voxels) and the chunk's weights for all 27 taps are
-// staged once in shared memory, and the A operand of tap t is read by
-// ldmatrix straight from the halo with per-lane row addresses, so each input
-// voxel is fetched once per chunk instead of once per tap.  Same result
-// definition as k_conv3d (the FP32 summation runs chunk-major).
-template <int BN>
-__global__ void __launch_bounds__(128) k_conv3d_box(const bf16 *__restrict__ in, int ics, int ic0,
-                                                    int cin, const bf16 *__restrict__ w,
-                                                    const float *__restrict__ bias, bf16 *out, int ocs,
-                                                    int oc0, int cout, Vol g, int bz, int by, int bx,
-                                                    int flags) {
+// conv3d on boxes of BZ x 8 x 8 voxels: warp z owns one plane of the box (64
+// voxels, four MMA row tiles) and BN output channels.  For every 16-channel chunk
+// the box's halo is staged once, in planes of 8 channels (16-byte rows: eight
+// consecutive voxels fill the 32 banks at any tap's shift), and the A operand of
+// a tap is read from it by ldmatrix at a constant offset.  CTAs are persistent:
+// the next chunk (or box) is copied while this one computes, and the weights stay
+// in shared memory for all boxes when they fit (WRES), else each chunk brings its
+// own.  Voxels outside the volume are zeros; outputs outside it are not stored.
+// Same sums as k_conv3d, chunk by chunk (the order of the kernel before).
+// Bound: mma.sync (half of its 550 TFLOP/s) and the shared-memory reads beside it,
+// four A and BN / 16 B fragments for BN / 2 mma.  48 -> 16 channels, 8 x 64^3: 283
+// us, 310 TFLOP/s; 605 us by the kernel before, which staged halo and weights for
+// 128 voxels at a time with nothing under way meanwhile.
+template <int BN, int BZ> struct BoxShape {
+    static constexpr int NT = 32 * BZ, ROWS = (BZ + 2) * 100, HBYTES = 2 * ROWS * 16, WBYTES = 27 * BN * 32;
+};
+template <int BN, int BZ, bool WRES>
+__global__ void __launch_bounds__(32 * BZ, BN == 16 ? 16 / BZ : BZ == 8 || BN == 64 ? 1 : 2) k_conv3d_box(const bf16 *__restrict__ in, int ics, int ic0, int cin,
+                                                        const bf16 *__restrict__ w, const float *__restrict__ bias,
+                                                        bf16 *out, int ocs, int oc0, Vol g, int nbx, int nby, int nbz,
+                                                        int nboxes, int flags) {
+    typedef BoxShape<BN, BZ> S;
+    constexpr int NT = S::NT, LT = NT / 20, NL = ((BZ + 2) * 10 + LT - 1) / LT;
+    constexpr int STAGE = S::HBYTES + (WRES ? 0 : S::WBYTES);
     extern __shared__ __align__(128) unsigned char dyn[];
-    const int hz = bz + 2, hy = by + 2, hx = bx + 2, nh = hz * hy * hx;
-    unsigned char *sa = dyn;                 // nh rows of 32 bytes
-    unsigned char *sb = dyn + nh * 32;       // 27 * BN rows of 32 bytes
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // box origin
-    const int nbx = g.w / bx, nby = g.h / by, nbz = g.d / bz;
-    int q = blockIdx.x;
-    const int ix = q % nbx; q /= nbx;
-    const int iy = q % nby; q /= nby;
-    const int iz = q % nbz;
-    const int b = q / nbz;
-    const int x0 = ix * bx, y0 = iy * by, z0 = iz * bz;
-    const int n0 = blockIdx.y * BN;
-    const int kc = cin / 16;
-
-    float acc[2][BN / 8][4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < BN / 8; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
-
-    // halo row of this lane's A rows, relative to the tap offset (0,0,0)
-    int hrow[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const int m = warp * 32 + i * 16 + (lane & 15);
-        const int mx = m % bx, my = (m / bx) % by, mz = m / (bx * by);
-        hrow[i] = (mz * hy + my) * hx + mx;
-    }
-    for (int c = 0; c < kc; ++c) {
-        const int cb = c * 16;
-        __syncthreads();  // the previous chunk's reads are done
-        for (int r = tid; r < nh * 2; r += 128) {
-            const int hrw = r >> 1, hh = r & 1;
-            const int lx = hrw % hx, ly = (hrw / hx) % hy, lz = hrw / (hx * hy);
-            const int gx = x0 + lx - 1, gy = y0 + ly - 1, gz = z0 + lz - 1;
-            const bool inside = (unsigned)gx < (unsigned)g.w && (unsigned)gy < (unsigned)g.h &&
-                                (unsigned)gz < (unsigned)g.d;
-            const i64 v = inside ? (((i64)b * g.d + gz) * g.h + gy) * g.w + gx : 0;
-            cp16(sa + sw32(hrw, hh), in + v * ics + ic0 + cb + hh * 8, inside ? 16u : 0u);
-        }
-        for (int r = tid; r < 27 * BN * 2; r += 128) {
-            const int row = r >> 1, hh = r & 1;  // row = t * BN + n
-            const int t = row / BN, nn = row % BN;
-            cp16(sb + sw32(row, hh), w + ((i64)(n0 + nn) * 27 + t) * cin + cb + hh * 8, 16u);
-        }
-        cp_commit();
-        cp_wait<0>();
-        __syncthreads();
-#pragma unroll 1
-        for (int t = 0; t < 27; ++t) {
-            const int toff = ((t / 9) * hy + (t / 3) % 3) * hx + t % 3;
-            unsigned a[2][4];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) ldm_x4(a[i], sa + sw32(hrow[i] + toff, lane >> 4));
-#pragma unroll
-            for (int j = 0; j < BN / 16; ++j) {
-                const int r = t * BN + j * 16 + (lane & 7) + ((lane >> 4) << 3);
-                unsigned bq[4];
-                ldm_x4(bq, sb + sw32(r, (lane >> 3) & 1));
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    mma16816(acc[i][2 * j], a[i], bq[0], bq[1]);
-                    mma16816(acc[i][2 * j + 1], a[i], bq[2], bq[3]);
-                }
-            }
-        }
-    }
-    const bool relu = flags & 1, accum = flags & 2, f32out = flags & 4;
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < BN / 8; ++j)
-#pragma unroll
-            for (int hr = 0; hr < 2; ++hr) {
-                const int m = warp * 32 + i * 16 + (lane >> 2) + hr * 8;
-                const int mx = m % bx, my = (m / bx) % by, mz = m / (bx * by);
-                const i64 v = (((i64)b * g.d + z0 + mz) * g.h + y0 + my) * g.w + x0 + mx;
-                const int n = n0 + j * 8 + 2 * (lane & 3);
-                float y0v = acc[i][j][2 * hr], y1v = acc[i][j][2 * hr + 1];
-                if (bias) {
-                    y0v += bias[n];
-                    y1v += bias[n + 1];
-                }
-                if (relu) {
-                    y0v = fmaxf(y0v, 0.f);
-                    y1v = fmaxf(y1v, 0.f);
-                }
-                if (f32out) {
-                    float2 *pf = reinterpret_cast<float2 *>(reinterpret_cast<float *>(out) + v * ocs + oc0 + n);
-                    if (accum) {
-                        const float2 o = *pf;
-                        y0v += o.x;
-                        y1v += o.y;
-                    }
-                    *pf = make_float2(y0v, y1v);
-                    continue;
-                }
-                __nv_bfloat162 *po = reinterpret_cast<__nv_bfloat162 *>(out + v * ocs + oc0 + n);
-                if (accum) {
-                    const float2 o = __bfloat1622float2(*po);
-                    y0v += o.x;
-                    y1v += o.y;
-                }
-                *po = __floats2bfloat162_rn(y0v, y1v);
-            }
-}
-
-// wgrad: dw[co][t][ci] += sum over the CTA's voxel slice of g[p][co] * in[p + off(t)][ci]
-// grid (slices, 27, cin/16); 4 warps split the slice, then reduce in shared memory.
-template <int CO>
-__global__ void __launch_bounds__(128) k_wgrad(const bf16 *__restrict__ in, int ics, int ic0,
-                                               int cin, const bf16 *__restrict__ gr, int gcs,
-                                               int gc0, float *dw, Vol g, int slice) {
-    constexpr int KS = 64;             // voxels per staged step (16 per warp)
-    constexpr int NCH = CO / 8;        // 16-byte chunks per gradient row
-    __shared__ __align__(128) unsigned char sg[2][KS * CO * 2];
-    __shared__ __align__(128) unsigned char si[2][KS * 32];
-    __shared__ float red[4][256];  // partial sums of warps 1..3, one 16-row group at a time
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int t = blockIdx.y, cb = blockIdx.z * 16;
-    const i64 nvox = g.count();
-    const i64 p0 = (i64)blockIdx.x * slice, p1 = min(nvox, p0 + slice);
-    const int nsteps = (int)((p1 - p0 + KS - 1) / KS);
-
-    auto stage = [&](int st, int s) {
-        const i64 pb = p0 + (i64)st * KS;
-        for (int q = tid; q < KS * NCH; q += 128) {
-            const int r = q / NCH, ch = q % NCH;
-            const i64 p = pb + r;
-            const bool ok = p < p1;
-            cp16(&sg[s][swn(r, ch, NCH)], gr + (ok ? p : 0) * gcs + gc0 + ch * 8, ok ? 16u : 0u);
-        }
-        for (int q = tid; q < KS * 2; q += 128) {
-            const int r = q >> 1, hh = q & 1;
-            const i64 p = pb + r;
-            const i64 src = p < p1 ? nbr(g, p, t) : -1;
-            cp16(&si[s][sw32(r, hh)], in + (src < 0 ? 0 : src) * ics + ic0 + cb + hh * 8,
-                 src < 0 ? 0u : 16u);
+    const int kc = cin / 16, n0 = blockIdx.y * BN;
+    unsigned char *stg = dyn + (WRES ? kc * S::WBYTES : 0);
+    // weights of chunk c, [tap][half][n] rows of 16 bytes
+    auto weights = [&](int c, unsigned char *dst) {
+        for (int p = tid; p < 27 * BN * 2; p += NT) {
+            const int hh = p & 1, n = (p >> 1) % BN, t = (p >> 1) / BN;
+            cp16(dst + ((t * 2 + hh) * BN + n) * 16, w + ((i64)(n0 + n) * 27 + t) * cin + c * 16 + hh * 8, 16u);
         }
     };
-
-    float acc[CO / 16][2][4];
+    if (WRES)
+        for (int c = 0; c < kc; ++c) weights(c, dyn + c * S::WBYTES);
+    // halo pieces of this thread: half and x fixed, lines (y, z) LT apart.  A line's
+    // offset and the faces of the box's halo it lies on are tabled once; a box
+    // whose halo crosses the volume's boundary leaves those faces out.
+    const int hh = tid & 1, hx = (tid >> 1) % 10, hl = tid / 20;
+    const bool loader = tid < LT * 20;
+    __shared__ int2 s_line[NL * LT];
+    for (int k = tid; k < NL * LT; k += NT) {
+        const int z = k / 10, y = k % 10;
+        s_line[k] = k < (BZ + 2) * 10 ? make_int2((z * g.h + y) * g.w * ics, (y == 0) | (y == 9) << 1 | (z == 0) << 2 | (z == BZ + 1) << 3)
+                                      : make_int2(0, 64);
+    }
+    const int fx = (hx == 0) << 4 | (hx == 9) << 5;
+    const bool whole = g.w % 8 == 0 && g.h % 8 == 0 && g.d % BZ == 0;  // no box reaches past the volume by more than its halo
+    __syncthreads();
+    int sx = 0, sy = 0, sz = 0;  // origin of the staged box's halo
+    i64 sb = 0;                  // first plane of its volume
+    auto stage = [&](int box, int c, int s) {
+        if (c == 0) {
+            int q = box;
+            sx = (q % nbx) * 8 - 1;
+            q /= nbx;
+            sy = (q % nby) * 8 - 1;
+            q /= nby;
+            sz = (q % nbz) * BZ - 1;
+            sb = (i64)(q / nbz) * g.d;
+        }
+        unsigned char *sh = stg + s * STAGE;
+        if (!WRES) weights(c, sh + S::HBYTES);
+        if (loader) {
+            const bf16 *src = in + (((sb + sz) * g.h + sy) * g.w + sx + hx) * ics + ic0 + c * 16 + hh * 8;
+            unsigned char *dst = sh + hh * (S::ROWS * 16) + hx * 16 + hl * 160;
+            if (whole) {
+                const int out_ = ((sy < 0) | (sy + 10 > g.h) << 1 | (sz < 0) << 2 | (sz + BZ + 2 > g.d) << 3 | (sx < 0) << 4 |
+                                  (sx + 10 > g.w) << 5);
 #pragma unroll
-    for (int m = 0; m < CO / 16; ++m)
+                for (int k = 0; k < NL; ++k) {
+                    const int2 ln = s_line[hl + k * LT];
+                    const bool ok = ((ln.y | fx) & out_) == 0;
+                    if (ln.y < 64) cp16(dst + k * LT * 160, ok ? src + ln.x : in, ok ? 16u : 0u);
+                }
+            } else {
+                const bool okx = (unsigned)(sx + hx) < (unsigned)g.w;
 #pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) acc[m][j][e] = 0.f;
-
-    if (nsteps > 0) stage(0, 0);
-    cp_commit();
-    for (int st = 0; st < nsteps; ++st) {
-        if (st + 1 < nsteps) stage(st + 1, (st + 1) & 1);
+                for (int k = 0; k < NL; ++k) {
+                    const int ln = hl + k * LT, z = ln / 10, y = ln - 10 * z;
+                    if (ln < (BZ + 2) * 10) {
+                        const bool ok = okx && (unsigned)(sy + y) < (unsigned)g.h && (unsigned)(sz + z) < (unsigned)g.d;
+                        cp16(dst + k * LT * 160, ok ? src + ((i64)z * g.h + y) * g.w * ics : in, ok ? 16u : 0u);
+                    }
+                }
+            }
+        }
         cp_commit();
-        cp_wait<1>();
-        __syncthreads();
-        const int s = st & 1;
-        const int rb = warp * 16;  // this warp's 16 voxels of the step
-        // B fragments (k = voxels, n = ci): trans loads of [p][ci]
-        unsigned bq[4];
-        {
-            const int r = rb + (lane & 7) + (((lane >> 3) & 1) << 3);
-            ldm_x4_t(bq, &si[s][sw32(r, lane >> 4)]);
+    };
+    const unsigned base0 = smem_u32(stg), wbase = WRES ? smem_u32(dyn) : base0 + S::HBYTES;
+    // this lane's rows: A (voxel lane & 15 of a tile, half lane >> 4), B (output
+    // channel, half)
+    const unsigned aa = (unsigned)((lane >> 4) * (S::ROWS * 16) + (warp * 100 + ((lane >> 3) & 1) * 10 + (lane & 7)) * 16);
+    const unsigned ba = (unsigned)(((lane >> 3) & 1) * (BN * 16) + ((lane & 7) + ((lane >> 4) << 3)) * 16);
+    const bool relu = flags & 1, accum = flags & 2, f32out = flags & 4;
+    int box = blockIdx.x, s = 0;
+    if (box < nboxes) stage(box, 0, 0);
+    for (; box < nboxes; box += gridDim.x) {
+        float acc[4][BN / 8][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < BN / 8; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[i][j][e] = 0.f;
+        for (int c = 0; c < kc; ++c, s ^= 1) {
+            if (c + 1 < kc) stage(box, c + 1, s ^ 1);
+            else if (box + (int)gridDim.x < nboxes) stage(box + gridDim.x, 0, s ^ 1);
+            else cp_commit();
+            cp_wait<1>();
+            __syncthreads();
+            const unsigned ab = base0 + (unsigned)(s * STAGE) + aa;
+            const unsigned bb = wbase + (unsigned)(WRES ? c * S::WBYTES : s * STAGE) + ba;
+            // a tap's fragments are read while the one before multiplies (at 64
+            // output channels the accumulators leave no registers for that, and
+            // 32 mma a tap hide the reads)
+            constexpr int NB = BN == 64 ? 1 : 2;
+            unsigned a[NB][4][4], bq[NB][BN / 16][4];
+            auto frag = [&](int t, unsigned(&af)[4][4], unsigned(&bf)[BN / 16][4]) {
+                const unsigned at = ab + (unsigned)(((t / 9) * 100 + (t / 3) % 3 * 10 + t % 3) * 16);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) ldm_x4_a(af[i], at + (unsigned)(i * 20 * 16));
+#pragma unroll
+                for (int j = 0; j < BN / 16; ++j) ldm_x4_a(bf[j], bb + (unsigned)(t * BN * 32 + j * 256));
+            };
+            if (NB == 2) frag(0, a[0], bq[0]);
+#pragma unroll
+            for (int t = 0; t < 27; ++t) {
+                const int u = t & (NB - 1);
+                if (NB == 1) frag(t, a[0], bq[0]);
+                else if (t + 1 < 27) frag(t + 1, a[u ^ 1], bq[u ^ 1]);
+#pragma unroll
+                for (int j = 0; j < BN / 16; ++j)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        mma16816(acc[i][2 * j], a[u][i], bq[u][j][0], bq[u][j][1]);
+                        mma16816(acc[i][2 * j + 1], a[u][i], bq[u][j][2], bq[u][j][3]);
+                    }
+            }
+            __syncthreads();
+        }
+        int q = box;
+        const int x0 = (q % nbx) * 8;
+        q /= nbx;
+        const int y0 = (q % nby) * 8;
+        q /= nby;
+        const int z = (q % nbz) * BZ + warp;
+        const i64 vb = (i64)(q / nbz) * g.d;
+        const int x = x0 + (lane >> 2);
+        const i64 o0 = (((vb + z) * g.h + y0) * g.w + x) * ocs + oc0 + n0 + 2 * (lane & 3);
+        const int rows = x < g.w && z < g.d ? min(8, g.h - y0) : 0, ystep = g.w * ocs;
+        if (!accum && !f32out) {
+#pragma unroll
+            for (int j = 0; j < BN / 8; ++j) {
+                const float b0 = bias ? __ldg(bias + n0 + j * 8 + 2 * (lane & 3)) : 0.f;
+                const float b1 = bias ? __ldg(bias + n0 + j * 8 + 2 * (lane & 3) + 1) : 0.f;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    float u = acc[i / 2][j][2 * (i & 1)], v = acc[i / 2][j][2 * (i & 1) + 1];
+                    if (bias) {
+                        u += b0;
+                        v += b1;
+                    }
+                    if (relu) {
+                        u = fmaxf(u, 0.f);
+                        v = fmaxf(v, 0.f);
+                    }
+                    if (i < rows)
+                        *reinterpret_cast<__nv_bfloat162 *>(out + o0 + (i64)i * ystep + j * 8) = __floats2bfloat162_rn(u, v);
+                }
+            }
+            continue;
         }
 #pragma unroll
-        for (int m = 0; m < CO / 16; ++m) {
-            // A fragment (m = co, k = voxels): trans loads of [p][co]
-            unsigned a[4];
-            const int r = rb + (lane & 7) + ((lane >> 4) << 3);
-            const int ch = m * 2 + ((lane >> 3) & 1);
-            ldm_x4_t(a, &sg[s][swn(r, ch, NCH)]);
-            mma16816(acc[m][0], a, bq[0], bq[1]);
-            mma16816(acc[m][1], a, bq[2], bq[3]);
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int hr = 0; hr < 2; ++hr) {
+                if (2 * i + hr >= rows) continue;
+                const i64 o = o0 + (i64)(2 * i + hr) * ystep;
+#pragma unroll
+                for (int j = 0; j < BN / 8; ++j) {
+                    const int n = n0 + j * 8 + 2 * (lane & 3);
+                    float y0v = acc[i][j][2 * hr], y1v = acc[i][j][2 * hr + 1];
+                    if (bias) {
+                        y0v += __ldg(bias + n);
+                        y1v += __ldg(bias + n + 1);
+                    }
+                    if (relu) {
+                        y0v = fmaxf(y0v, 0.f);
+                        y1v = fmaxf(y1v, 0.f);
+                    }
+                    if (f32out) {
+                        float2 *pf = reinterpret_cast<float2 *>(reinterpret_cast<float *>(out) + o + j * 8);
+                        if (accum) {
+                            const float2 ov = *pf;
+                            y0v += ov.x;
+                            y1v += ov.y;
+                        }
+                        *pf = make_float2(y0v, y1v);
+                        continue;
+                    }
+                    __nv_bfloat162 *po = reinterpret_cast<__nv_bfloat162 *>(out + o + j * 8);
+                    if (accum) {
+                        const float2 ov = __bfloat1622float2(*po);
+                        y0v += ov.x;
+                        y1v += ov.y;
+                    }
+                    *po = __floats2bfloat162_rn(y0v, y1v);
+                }
+            }
+    }
+    cp_wait<0>();
+}
+
+// wgrad: dw[co][t][ci] += sum over the CTA's boxes of g[p][co] * in[p + off(t)][ci]
+// for one 16-channel chunk of ci and CO output channels, all 27 taps at once.  A
+// box is 2 x 8 x 8 voxels; its gradients and the chunk's halo (4 x 10 x 10 voxels)
+// are staged once, in planes of 8 channels (16-byte rows: eight consecutive
+// voxels fill the 32 banks, at any tap's shift, without a swizzle), while the
+// box before computes.  The eight warps share the taps (warp w: w, w + 8, ..), so
+// a fragment of the gradient serves 3 or 4 taps, and every partial sum stays in
+// registers until the CTA's boxes are done (FP32 atomics, one per CTA and
+// weight).  Voxels outside the volume are zeros on both sides.
+// Bound: mma.sync (54 % of its cycles) and the fragments' latency.  cin 96, cout
+// 32, 4 x 32^3: 90 us, 240 TFLOP/s; 569 us by the kernel before, which staged the
+// gradient and a shifted input once per tap and chunk.
+constexpr int WG_HALO = 4 * 10 * 10, WG_VOX = 128;
+template <int CO> struct WgradShape {
+    static constexpr int GBYTES = (CO / 8) * WG_VOX * 16, HBYTES = 2 * WG_HALO * 16, STAGE = GBYTES + HBYTES;
+};
+template <int CO>
+__global__ void __launch_bounds__(256, CO == 64 ? 1 : 2) k_wgrad(const bf16 *__restrict__ in, int ics, int ic0, int cin,
+                                                                 const bf16 *__restrict__ gr, int gcs, int gc0,
+                                                                 float *dw, Vol g, int nbx, int nby, int nbz,
+                                                                 int nboxes) {
+    typedef WgradShape<CO> S;
+    extern __shared__ __align__(128) unsigned char dyn[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int cb = blockIdx.y * 16, o0 = blockIdx.z * CO;
+    // 16-byte pieces of this thread, the same of every box: halo piece p is half
+    // p & 1 of halo voxel p >> 1, gradient piece p channels 8 (p % (CO / 8)) .. of
+    // box voxel p / (CO / 8); offsets from the box's origin and, for the halo, the
+    // faces it lies on
+    constexpr int NH = (2 * WG_HALO + 255) / 256, NG = CO / 8 * WG_VOX / 256;
+    int ho[NH], hf[NH], go[NG];
+    auto halo_at = [&](int k, int &x, int &y, int &z) {
+        const int v = (tid + 256 * k) >> 1;
+        x = v % 10 - 1;
+        y = v / 10 % 10 - 1;
+        z = v / 100 - 1;
+        return v < WG_HALO;
+    };
+    auto grad_at = [&](int k, int &x, int &y, int &z) {
+        const int v = (tid + 256 * k) / (CO / 8);
+        x = v & 7;
+        y = v >> 3 & 7;
+        z = v >> 6;
+    };
+#pragma unroll
+    for (int k = 0; k < NH; ++k) {
+        int x, y, z;
+        const bool on = halo_at(k, x, y, z);
+        ho[k] = ((z * g.h + y) * g.w + x) * ics + (tid & 1) * 8;
+        hf[k] = on ? (x < 0) | (x == 8) << 1 | (y < 0) << 2 | (y == 8) << 3 | (z < 0) << 4 | (z == 2) << 5 : 64;
+    }
+#pragma unroll
+    for (int k = 0; k < NG; ++k) {
+        int x, y, z;
+        grad_at(k, x, y, z);
+        go[k] = ((z * g.h + y) * g.w + x) * gcs + (tid + 256 * k) % (CO / 8) * 8;
+    }
+    const bool whole = g.w % 8 == 0 && g.h % 8 == 0 && g.d % 2 == 0;
+    auto stage = [&](int box, int s) {
+        int q = box;
+        const int x0 = (q % nbx) * 8;
+        q /= nbx;
+        const int y0 = (q % nby) * 8;
+        q /= nby;
+        const int z0 = (q % nbz) * 2;
+        const i64 v0 = (((i64)(q / nbz) * g.d + z0) * g.h + y0) * g.w + x0;
+        unsigned char *sg = dyn + s * S::STAGE, *sh = sg + S::GBYTES + (tid & 1) * (WG_HALO * 16) + (tid >> 1) * 16;
+        const bf16 *pi = in + v0 * ics + ic0 + cb, *pg = gr + v0 * gcs + gc0 + o0;
+        unsigned char *dg = sg + tid % (CO / 8) * (WG_VOX * 16) + tid / (CO / 8) * 16;  // 256 is a multiple of CO / 8
+        if (whole) {
+            const int out_ = (x0 == 0) | (x0 + 8 == g.w) << 1 | (y0 == 0) << 2 | (y0 + 8 == g.h) << 3 | (z0 == 0) << 4 |
+                             (z0 + 2 == g.d) << 5;
+#pragma unroll
+            for (int k = 0; k < NH; ++k) {
+                const bool ok = (hf[k] & out_) == 0;
+                if (hf[k] < 64) cp16(sh + k * 128 * 16, ok ? pi + ho[k] : in, ok ? 16u : 0u);
+            }
+#pragma unroll
+            for (int k = 0; k < NG; ++k) cp16(dg + k * (256 / (CO / 8)) * 16, pg + go[k], 16u);
+        } else {
+#pragma unroll
+            for (int k = 0; k < NH; ++k) {
+                int x, y, z;
+                halo_at(k, x, y, z);
+                const bool ok = (unsigned)(x0 + x) < (unsigned)g.w && (unsigned)(y0 + y) < (unsigned)g.h &&
+                                (unsigned)(z0 + z) < (unsigned)g.d;
+                if (hf[k] < 64) cp16(sh + k * 128 * 16, ok ? pi + ho[k] : in, ok ? 16u : 0u);
+            }
+#pragma unroll
+            for (int k = 0; k < NG; ++k) {
+                int x, y, z;
+                grad_at(k, x, y, z);
+                const bool ok = x0 + x < g.w && y0 + y < g.h && z0 + z < g.d;
+                cp16(dg + k * (256 / (CO / 8)) * 16, ok ? pg + go[k] : gr, ok ? 16u : 0u);
+            }
+        }
+        cp_commit();
+    };
+    float acc[4][CO / 16][2][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int m = 0; m < CO / 16; ++m)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[j][m][h][e] = 0.f;
+    // this lane's addresses inside a stage: gradient rows and, per tap, halo rows
+    const unsigned ga = (unsigned)((((lane >> 3) & 1) * WG_VOX + (lane & 7) + ((lane >> 4) << 3)) * 16);
+    unsigned ha[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int t = min(warp + 8 * j, 26);
+        // voxel of this lane in a group of 16: x = lane & 7, y = lane >> 3 & 1
+        const int row = ((t / 9) * 10 + (t / 3) % 3 + ((lane >> 3) & 1)) * 10 + t % 3 + (lane & 7);
+        ha[j] = (unsigned)(S::GBYTES + (lane >> 4) * (WG_HALO * 16) + row * 16);
+    }
+    const int taps = warp < 3 ? 4 : 3;
+    int box = blockIdx.x, s = 0;
+    if (box < nboxes) stage(box, 0);
+    for (; box < nboxes; box += gridDim.x, s ^= 1) {
+        if (box + (int)gridDim.x < nboxes) stage(box + gridDim.x, s ^ 1);
+        else cp_commit();
+        cp_wait<1>();
+        __syncthreads();
+        const unsigned base = smem_u32(dyn) + (unsigned)(s * S::STAGE);
+        // 16 voxels a step: two rows of 8 in plane z = k / 4; the next tap's
+        // fragment is read while this one multiplies
+        unsigned a[CO / 16][4], bq[2][4];
+        ldm_x4_ta(bq[0], base + ha[0]);
+        const bool low = box / nbx % nby * 8 + 4 >= g.h;  // the box's rows y >= 4 lie outside: zeros
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            if ((k & 3) >= 2 && low) continue;
+#pragma unroll
+            for (int m = 0; m < CO / 16; ++m) ldm_x4_ta(a[m], base + ga + (unsigned)((2 * m * WG_VOX + 16 * k) * 16));
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int kn = j == 3 ? k + 1 : k, jn = (j + 1) & 3;  // what follows (tap 3 repeats tap 26 on five warps)
+                if (j == 3 && (k & 3) == 1 && low) ldm_x4_ta(bq[0], base + ha[0] + (unsigned)((k / 4 + 1) % 2 * 1600));
+                else if (kn < 8) ldm_x4_ta(bq[(j + 1) & 1], base + ha[jn] + (unsigned)(((kn / 4) * 100 + (kn % 4) * 20) * 16));
+                if (j == 3 && taps == 3) continue;
+#pragma unroll
+                for (int m = 0; m < CO / 16; ++m) {
+                    mma16816(acc[j][m][0], a[m], bq[j & 1][0], bq[j & 1][1]);
+                    mma16816(acc[j][m][1], a[m], bq[j & 1][2], bq[j & 1][3]);
+                }
+            }
         }
         __syncthreads();
     }
     cp_wait<0>();
-    // reduce the 4 warps' partial sums: warps 1..3 write, warp 0 adds, 16 co rows at a time
-    float *dwt = dw + (i64)t * cin + cb;  // dw[co][t][ci] = dwt[co*27*cin + ci]
+    const bool pairs = reinterpret_cast<uintptr_t>(dw) % 8 == 0;
 #pragma unroll
-    for (int m = 0; m < CO / 16; ++m) {
-        __syncthreads();
-        if (warp > 0)
+    for (int j = 0; j < 4; ++j) {
+        if (j == 3 && taps == 3) break;
+        float *dwt = dw + (i64)(warp + 8 * j) * cin + cb;  // dw[co][t][ci] = dwt[co * 27 * cin + ci]
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
+        for (int m = 0; m < CO / 16; ++m)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) red[warp][(j * 4 + e) * 32 + lane] = acc[m][j][e];
-        __syncthreads();
-        if (warp == 0) {
+            for (int h = 0; h < 2; ++h)
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    float v = acc[m][j][e] + red[1][(j * 4 + e) * 32 + lane] +
-                              red[2][(j * 4 + e) * 32 + lane] + red[3][(j * 4 + e) * 32 + lane];
-                    const int co = m * 16 + (lane >> 2) + (e >> 1) * 8;
-                    const int ci = j * 8 + 2 * (lane & 3) + (e & 1);
-                    atomicAdd(dwt + (i64)co * 27 * cin + ci, v);
+                for (int e = 0; e < 4; e += 2) {
+                    const int co = o0 + m * 16 + (lane >> 2) + (e >> 1) * 8, ci = h * 8 + 2 * (lane & 3);
+                    float *p = dwt + (i64)co * 27 * cin + ci;
+                    if (pairs) {
+                        asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(acc[j][m][h][e]), "f"(acc[j][m][h][e + 1]) : "memory");
+                    } else {
+                        atomicAdd(p, acc[j][m][h][e]);
+                        atomicAdd(p + 1, acc[j][m][h][e + 1]);
+                    }
                 }
-        }
     }
 }
 
@@ -463,28 +620,6 @@ __global__ void k_weight_flip(const bf16 *__restrict__ w, bf16 *__restrict__ wt,
         const int t = (int)(r % 27), co = (int)(r / 27);
         wt[((i64)ci * 27 + (26 - t)) * cout + co] = w[q];
     }
-}
-
-// g[p][gc0 + c] *= (act[p][ac0 + c] > 0)
-__global__ void k_relu_bwd(bf16 *g, int gcs, int gc0, const bf16 *__restrict__ act, int acs, int ac0,
-                           int c, i64 nvox) {
-    const i64 total = nvox * c;
-    for (i64 q = (i64)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (i64)gridDim.x * blockDim.x) {
-        const i64 p = q / c;
-        const int k = (int)(q % c);
-        if (!(__bfloat162float(act[p * acs + ac0 + k]) > 0.f)) g[p * gcs + gc0 + k] = __float2bfloat16(0.f);
-    }
-}
-
-// db[c] += sum_p g[p][gc0 + c]; one thread per channel and voxel slice
-__global__ void k_bias_grad(const bf16 *__restrict__ g, int gcs, int gc0, int c, i64 nvox,
-                            i64 slice, float *db) {
-    const int k = threadIdx.x % c;
-    const int lanes = blockDim.x / c;
-    const i64 p0 = (i64)blockIdx.x * slice, p1 = min(nvox, p0 + slice);
-    float s = 0.f;
-    for (i64 p = p0 + threadIdx.x / c; p < p1; p += lanes) s += __bfloat162float(g[p * gcs + gc0 + k]);
-    atomicAdd(db + k, s);
 }
 
 // Elementwise volume kernels work on groups of 8 channels (16 bytes), which
@@ -510,6 +645,71 @@ __device__ __forceinline__ void st8(bf16 *p, const Oct &o) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) h[k] = __floats2bfloat162_rn(o.v[2 * k], o.v[2 * k + 1]);
     *reinterpret_cast<uint4 *>(p) = u;
+}
+
+// g[p][gc0 + c] *= (act[p][ac0 + c] > 0), 8 channels a thread
+__global__ void k_relu_bwd(bf16 *g, int gcs, int gc0, const bf16 *__restrict__ act, int acs, int ac0,
+                           int c8, i64 nvox) {
+    const i64 total = nvox * c8;
+    for (i64 q = (i64)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (i64)gridDim.x * blockDim.x) {
+        const i64 p = q / c8;
+        const int k = (int)(q - p * c8) * 8;
+        bf16 *pg = g + p * gcs + gc0 + k;
+        uint4 w = *reinterpret_cast<const uint4 *>(pg);
+        const uint4 av = *reinterpret_cast<const uint4 *>(act + p * acs + ac0 + k);
+        const __nv_bfloat16 *ah = reinterpret_cast<const __nv_bfloat16 *>(&av);
+        __nv_bfloat16 *gh = reinterpret_cast<__nv_bfloat16 *>(&w);
+#pragma unroll
+        for (int e = 0; e < 8; ++e)
+            if (!(__bfloat162float(ah[e]) > 0.f)) gh[e] = __float2bfloat16(0.f);
+        *reinterpret_cast<uint4 *>(pg) = w;
+    }
+}
+// the same for channel counts, offsets or strides that are not multiples of 8
+__global__ void k_relu_bwd1(bf16 *g, int gcs, int gc0, const bf16 *__restrict__ act, int acs, int ac0,
+                            int c, i64 nvox) {
+    const i64 total = nvox * c;
+    for (i64 q = (i64)blockIdx.x * blockDim.x + threadIdx.x; q < total; q += (i64)gridDim.x * blockDim.x) {
+        const i64 p = q / c;
+        const int k = (int)(q % c);
+        if (!(__bfloat162float(act[p * acs + ac0 + k]) > 0.f)) g[p * gcs + gc0 + k] = __float2bfloat16(0.f);
+    }
+}
+
+// db[c] += sum_p g[p][gc0 + c]: a thread sums 8 channels over its voxels of the
+// block's slice, the block's sums meet in shared memory, one atomic per channel
+__global__ void __launch_bounds__(256) k_bias_grad(const bf16 *__restrict__ g, int gcs, int gc0, int c8, i64 nvox,
+                                                   i64 slice, float *db) {
+    __shared__ float red[256][9];
+    const int tid = threadIdx.x, k = tid % c8, lanes = 256 / c8;
+    const i64 p0 = (i64)blockIdx.x * slice, p1 = min(nvox, p0 + slice);
+    float s[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s[e] = 0.f;
+#pragma unroll 4
+    for (i64 p = p0 + tid / c8; p < p1; p += lanes) {
+        const Oct o = ld8(g + p * gcs + gc0 + k * 8);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s[e] += o.v[e];
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) red[tid][e] = s[e];
+    __syncthreads();
+    if (tid < c8 * 8) {
+        float t = 0.f;
+        for (int r = 0; r < lanes; ++r) t += red[r * c8 + tid / 8][tid % 8];
+        atomicAdd(db + tid, t);
+    }
+}
+// the same for channel counts, offsets or strides that are not multiples of 8
+__global__ void k_bias_grad1(const bf16 *__restrict__ g, int gcs, int gc0, int c, i64 nvox,
+                             i64 slice, float *db) {
+    const int k = threadIdx.x % c;
+    const int lanes = blockDim.x / c;
+    const i64 p0 = (i64)blockIdx.x * slice, p1 = min(nvox, p0 + slice);
+    float s = 0.f;
+    for (i64 p = p0 + threadIdx.x / c; p < p1; p += lanes) s += __bfloat162float(g[p * gcs + gc0 + k]);
+    atomicAdd(db + k, s);
 }
 
 // 2x2x2 average pooling of volume g (even sides): one thread per coarse voxel
@@ -900,6 +1100,38 @@ int last_err() {
     return 0;
 }
 
+// all weights stay in shared memory while two CTAs still fit an SM
+bool box_weights_resident(int bn, int kc) { return bn < 64 && kc * 27 * bn * 32 <= 56 * 1024; }
+
+// Output channels and depth of the box kernel's CTAs: the pair with the least
+// estimated time.  A tap of one warp takes bn cycles of the SM's tensor pipe and
+// 16 + bn / 4 of its shared memory, of which about a quarter overlap (measured:
+// 48 -> 16 channels at 8 x 64^3), and no less than the latency of its reads and
+// mma; every chunk is copied by the CTA's own threads.  Wide CTAs read less, narrow ones leave more warps on a small volume
+// (8 x 16^3, 64 -> 64: bn 64 58 us, 16 43 us; 8 x 8^3, 128 -> 128: 55 and 25 us).
+struct BoxPlan {
+    int bn, bz;
+    double t;  // SM cycles
+};
+BoxPlan box_plan(i64 plane, int d, int kc, int cout, int bn0) {
+    BoxPlan best{bn0, 8, 1e300};
+    for (int bn = bn0; bn >= 16; bn /= 2)
+        for (int bz = 8; bz >= 2; bz /= 2) {
+            const i64 tasks = plane * ((d + bz - 1) / bz) * (cout / bn);
+            const int halo = (bz + 2) * 100 * 32, wb = 27 * bn * 32;
+            const int sm = box_weights_resident(bn, kc) ? 2 * halo + kc * wb : 2 * (halo + wb);
+            const i64 fit = std::max(1, std::min(227 * 1024 / (sm + 2048), (bn == 16 ? 16 : 8) / bz));
+            const i64 rounds = (tasks + 148 * fit - 1) / (148 * fit);
+            const double warps = (double)std::min<i64>(fit, (tasks + 147) / 148) * bz;
+            const double tap = std::max(60.0 + 2.2 * bn, 0.75 * warps * (1.25 * bn + 16));
+            // a lone CTA on its SM has nobody to compute while it stages
+            const double copy = 500.0 + 20.0 / 16 * (halo + (box_weights_resident(bn, kc) ? 0 : wb)) / (32 * bz);
+            const double t = (double)rounds * kc * (27 * tap + copy) * (fit == 1 ? 1.25 : 1.0);
+            if (t < best.t * 0.98) best = {bn, bz, t};
+        }
+    return best;
+}
+
 bool ch_ok(int c) { return c > 0 && c % 16 == 0; }
 
 }  // namespace
@@ -914,36 +1146,51 @@ int xcnn_conv3d(const void *in, int ics, int ic0, int cin, const void *w, const 
     Vol g{nb, d, h, wd};
     const i64 nvox = (i64)nb * d * h * wd;
     cudaStream_t s = (cudaStream_t)stream;
-    const int bn = cout % 64 == 0 ? 64 : (cout % 32 == 0 ? 32 : 16);
+    const int bn0 = cout % 64 == 0 ? 64 : (cout % 32 == 0 ? 32 : 16);
     const bf16 *pi = (const bf16 *)in;
     const bf16 *pw = (const bf16 *)w;
     bf16 *po = (bf16 *)out;
     if (g_tc_conv) {
-        dim3 grid((unsigned)((nvox + BM - 1) / BM), (unsigned)(cout / bn));
-        if (bn == 64) k_conv3d_tc<64><<<grid, 128, 0, s>>>(pi, ics, ic0, cin, pw, bias, po, ocs, oc0, cout, g, flags);
-        else if (bn == 32) k_conv3d_tc<32><<<grid, 128, 0, s>>>(pi, ics, ic0, cin, pw, bias, po, ocs, oc0, cout, g, flags);
+        dim3 grid((unsigned)((nvox + BM - 1) / BM), (unsigned)(cout / bn0));
+        if (bn0 == 64) k_conv3d_tc<64><<<grid, 128, 0, s>>>(pi, ics, ic0, cin, pw, bias, po, ocs, oc0, cout, g, flags);
+        else if (bn0 == 32) k_conv3d_tc<32><<<grid, 128, 0, s>>>(pi, ics, ic0, cin, pw, bias, po, ocs, oc0, cout, g, flags);
         else k_conv3d_tc<16><<<grid, 128, 0, s>>>(pi, ics, ic0, cin, pw, bias, po, ocs, oc0, cout, g, flags);
         return last_err();
     }
-    // box kernel when the volume tiles into 128-voxel boxes of at least 8 x 8
-    // in (y, x): sides multiples of 8 and a depth that is a multiple of 2
-    const int bx = 8, by = 8, bz = 2;
-    if (box_conv_enabled() && wd % bx == 0 && h % by == 0 && d % bz == 0) {
-        dim3 gb((unsigned)((i64)nb * (d / bz) * (h / by) * (wd / bx)), (unsigned)(cout / bn));
-        const int sm = (bz + 2) * (by + 2) * (bx + 2) * 32 + 27 * bn * 32;
-#define LB(BN)                                                                                     \
-    {                                                                                              \
-        auto k = k_conv3d_box<BN>;                                                                 \
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);                 \
-        k<<<gb, 128, sm, s>>>(pi, ics, ic0, cin, pw, bias, po, ocs, oc0, cout, g, bz, by, bx, flags); \
+    // box kernel unless padding the volume to boxes costs more than the
+    // voxel-tile kernel's steps (one per tap and chunk, about 700 cycles each
+    // while its tiles fill an SM up to three times)
+    auto up = [](int n, int m) { return (n + m - 1) / m; };
+    const i64 plane = (i64)nb * up(h, 8) * up(wd, 8);
+    const BoxPlan bp = box_plan(plane, d, cin / 16, cout, bn0);
+    const int bn = bp.bn, bz = bp.bz;
+    const i64 nboxes = plane * up(d, bz), tiles = (nvox + BM - 1) / BM * (cout / bn0);
+    if (box_conv_enabled() && nboxes <= 0x3fffffff && bp.t < 27.0 * (cin / 16) * 700.0 * (double)((tiles + 443) / 444) &&
+        (i64)10 * h * wd * ics <= 0x7fffffff && (i64)wd * ocs <= 0x7fffffff) {
+#define LB(BN, BZ, WRES)                                                                                            \
+    {                                                                                                               \
+        typedef BoxShape<BN, BZ> S;                                                                                 \
+        auto k = k_conv3d_box<BN, BZ, WRES>;                                                                        \
+        const int sm = WRES ? 2 * S::HBYTES + cin / 16 * S::WBYTES : 2 * (S::HBYTES + S::WBYTES);                   \
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);                                   \
+        int per = 0;                                                                                                \
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, S::NT, sm) != cudaSuccess || per < 1) per = 1;    \
+        dim3 gb((unsigned)std::max<i64>(1, std::min<i64>(nboxes, (i64)148 * per / (cout / bn))), (unsigned)(cout / bn)); \
+        k<<<gb, S::NT, sm, s>>>(pi, ics, ic0, cin, pw, bias, po, ocs, oc0, g, up(wd, 8), up(h, 8), up(d, bz), (int)nboxes, flags); \
     }
-        if (bn == 64) LB(64) else if (bn == 32) LB(32) else LB(16)
+#define LBZ(BN, WRES)                                                                                               \
+    if (bz == 8) LB(BN, 8, WRES) else if (bz == 4) LB(BN, 4, WRES) else LB(BN, 2, WRES)
+        const bool res = box_weights_resident(bn, cin / 16);
+        if (bn == 64) LBZ(64, false)
+        else if (bn == 32) { if (res) LBZ(32, true) else LBZ(32, false) }
+        else { if (res) LBZ(16, true) else LBZ(16, false) }
+#undef LBZ
 #undef LB
         return last_err();
     }
-    dim3 grid((unsigned)((nvox + BM - 1) / BM), (unsigned)(cout / bn));
-    if (bn == 64) k_conv3d<64><<<grid, 128, 0, s>>>(pi, ics, ic0, cin, pw, bias, po, ocs, oc0, cout, g, flags);
-    else if (bn == 32) k_conv3d<32><<<grid, 128, 0, s>>>(pi, ics, ic0, cin, pw, bias, po, ocs, oc0, cout, g, flags);
+    dim3 grid((unsigned)((nvox + BM - 1) / BM), (unsigned)(cout / bn0));
+    if (bn0 == 64) k_conv3d<64><<<grid, 128, 0, s>>>(pi, ics, ic0, cin, pw, bias, po, ocs, oc0, cout, g, flags);
+    else if (bn0 == 32) k_conv3d<32><<<grid, 128, 0, s>>>(pi, ics, ic0, cin, pw, bias, po, ocs, oc0, cout, g, flags);
     else k_conv3d<16><<<grid, 128, 0, s>>>(pi, ics, ic0, cin, pw, bias, po, ocs, oc0, cout, g, flags);
     return last_err();
 }
@@ -954,21 +1201,27 @@ int xcnn_conv3d_wgrad(const void *in, int ics, int ic0, int cin, const void *gra
         gc0 + cout > gcs || !(cout == 16 || cout == 32 || cout == 64 || cout == 128))
         return 2;
     Vol g{nb, d, h, wd};
-    const i64 nvox = (i64)nb * d * h * wd;
-    // slices of at least 512 voxels, about 4 CTAs per SM in total
-    const i64 want = (i64)148 * 4 / (27 * (cin / 16));
-    i64 slice = (nvox + (want > 1 ? want : 1) - 1) / (want > 1 ? want : 1);
-    slice = ((slice < 512 ? 512 : slice) + 63) / 64 * 64;
-    dim3 grid((unsigned)((nvox + slice - 1) / slice), 27, (unsigned)(cin / 16));
+    const int nbx = (wd + 7) / 8, nby = (h + 7) / 8, nbz = (d + 1) / 2;
+    const i64 nboxes = (i64)nb * nbx * nby * nbz;
+    if (nboxes > 0x3fffffff || (i64)3 * h * wd * std::max(ics, gcs) > 0x7fffffff) return 2;  // 32-bit offsets in a box
+    const int co = cout > 64 ? 64 : cout, nci = cin / 16, nco = cout / co;
+    // two CTAs per SM (one at 64 channels, whose partial sums fill the register
+    // file), shared out over the channel chunks; every CTA has a box
+    const i64 want = (i64)148 * (co == 64 ? 1 : 2) / (nci * nco);
+    const unsigned slices = (unsigned)std::max<i64>(0, want < 1 ? std::min<i64>(1, nboxes) : std::min(want, nboxes));
+    dim3 grid(slices, (unsigned)nci, (unsigned)nco);
     cudaStream_t s = (cudaStream_t)stream;
     const bf16 *pi = (const bf16 *)in;
     const bf16 *pg = (const bf16 *)grad;
-    switch (cout) {
-    case 16: k_wgrad<16><<<grid, 128, 0, s>>>(pi, ics, ic0, cin, pg, gcs, gc0, dw, g, (int)slice); break;
-    case 32: k_wgrad<32><<<grid, 128, 0, s>>>(pi, ics, ic0, cin, pg, gcs, gc0, dw, g, (int)slice); break;
-    case 64: k_wgrad<64><<<grid, 128, 0, s>>>(pi, ics, ic0, cin, pg, gcs, gc0, dw, g, (int)slice); break;
-    default: k_wgrad<128><<<grid, 128, 0, s>>>(pi, ics, ic0, cin, pg, gcs, gc0, dw, g, (int)slice); break;
+#define LW(CO)                                                                                                    \
+    {                                                                                                             \
+        auto k = k_wgrad<CO>;                                                                                     \
+        const int sm = 2 * WgradShape<CO>::STAGE;                                                                 \
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);                                 \
+        k<<<grid, 256, sm, s>>>(pi, ics, ic0, cin, pg, gcs, gc0, dw, g, nbx, nby, nbz, (int)nboxes);              \
     }
+    if (co == 16) LW(16) else if (co == 32) LW(32) else LW(64)
+#undef LW
     return last_err();
 }
 
@@ -980,16 +1233,27 @@ int xcnn_weight_flip(const void *w, void *wt, int cout, int cin, void *stream) {
 
 int xcnn_relu_bwd(void *g, int gcs, int gc0, const void *act, int acs, int ac0, int c, int64_t nvox,
                   void *stream) {
-    k_relu_bwd<<<grid_for(nvox * c), 256, 0, (cudaStream_t)stream>>>((bf16 *)g, gcs, gc0, (const bf16 *)act,
-                                                                        acs, ac0, c, nvox);
+    cudaStream_t s = (cudaStream_t)stream;
+    const bool wide = c % 8 == 0 && gcs % 8 == 0 && gc0 % 8 == 0 && acs % 8 == 0 && ac0 % 8 == 0 &&
+                      (uintptr_t)g % 16 == 0 && (uintptr_t)act % 16 == 0;
+    if (wide) k_relu_bwd<<<grid_for(nvox * (c / 8)), 256, 0, s>>>((bf16 *)g, gcs, gc0, (const bf16 *)act, acs, ac0, c / 8, nvox);
+    else k_relu_bwd1<<<grid_for(nvox * c), 256, 0, s>>>((bf16 *)g, gcs, gc0, (const bf16 *)act, acs, ac0, c, nvox);
     return last_err();
 }
 
 int xcnn_bias_grad(const void *g, int gcs, int gc0, int c, int64_t nvox, float *db, void *stream) {
     if (c <= 0 || c > 256 || 256 % c) return 2;
+    cudaStream_t s = (cudaStream_t)stream;
+    if (c % 8 == 0 && gcs % 8 == 0 && gc0 % 8 == 0 && (uintptr_t)g % 16 == 0 && nvox > 0) {
+        // slices of about 64 voxels a thread row, at most four blocks per SM
+        const i64 rows = 256 / (c / 8);
+        const i64 blocks = std::min<i64>(148 * 4, (nvox + rows * 16 - 1) / (rows * 16));
+        const i64 slice = (nvox + blocks - 1) / blocks;
+        k_bias_grad<<<(unsigned)((nvox + slice - 1) / slice), 256, 0, s>>>((const bf16 *)g, gcs, gc0, c / 8, nvox, slice, db);
+        return last_err();
+    }
     const i64 slice = 4096;
-    k_bias_grad<<<(unsigned)((nvox + slice - 1) / slice), 256, 0, (cudaStream_t)stream>>>(
-        (const bf16 *)g, gcs, gc0, c, nvox, slice, db);
+    k_bias_grad1<<<(unsigned)((nvox + slice - 1) / slice), 256, 0, s>>>((const bf16 *)g, gcs, gc0, c, nvox, slice, db);
     return last_err();
 }
 
