@@ -1458,6 +1458,9 @@ struct Krylov : Solver {
     bool seq_dot = false;    // dot_order = sequential
     DVec r0, r, p, v, s, t, p_, s_;
     DBuf part, sc;
+    DBuf grid;  // workspace of the iterations in one launch, its parts at goff
+    size_t goff[3] = {};
+    std::vector<double> hhist;
     Pinned hres;
     enum { RHO, S1, S2, S3, S4, ALPHA, OMEGA, BETA, C1, RES, AC, OC, ICONV, ONES, NALPHA, NOMEGA,
            THETA, PHI, PSI, ETA, DELTA, STAT, TOLS, NSC };
@@ -1491,6 +1494,7 @@ struct Krylov : Solver {
         hres.alloc(nv);
         hres_async.alloc(nv);
         XCUDA(cudaEventCreateWithFlags(&res_ready, cudaEventDisableTiming));
+        setup_grid(n);
     }
 
     const DCsr &dA() const { return A->d; }
@@ -1562,6 +1566,7 @@ struct Krylov : Solver {
         // The convergence masks are kept on the device; the host reads the
         // NV residuals once per iteration while the last two kernels run.
         const xk::BicgScalars sc = scalars();
+        if (grid.p && !seq_dot && !ktime_on() && solve_grid(x, sc, max_iters, st)) return;
         for (int it = 1;; ++it) {
             conv.iters = it;
             DVec *pp = &p, *ss = &s;
@@ -1606,6 +1611,54 @@ struct Krylov : Solver {
             if (it >= max_iters) break;
         }
         XCUDA(cudaStreamSynchronize(st));
+    }
+
+    // Without a preconditioner, systems whose iteration is launches and waits
+    // rather than work run whole iterations in one cooperative launch, up to
+    // GRID_ITERS of them.  Not while kernels are timed one by one.
+    static constexpr int GRID_ITERS = 256;
+    void setup_grid(i64 n) {
+        if (precond || reordered || cg || !xk::bicg_grid_fits(n)) return;
+        // one allocation: partials, residuals with {error flag, iterations run}
+        // behind them, the second buffers of p and v
+        const size_t vec = xk::bicg_grid_fly(prec, nv) ? (size_t)n * nv * prec_size(prec) : 0;
+        goff[0] = (xk::bicg_grid_bytes(n, nv) + 255) / 256 * 256;
+        goff[1] = goff[0] + (sizeof(double) * (GRID_ITERS * nv + 1) + 255) / 256 * 256;
+        goff[2] = goff[1] + (vec + 255) / 256 * 256;
+        grid.alloc(goff[2] + vec);
+        hhist.resize(GRID_ITERS * nv + 1);
+    }
+    // false: the device cannot hold the grid at once, nothing has run
+    bool solve_grid(DVec &x, const xk::BicgScalars &sc, int max_iters, cudaStream_t st) {
+        const DCsr &a = dA();
+        char *base = grid.as<char>();
+        XCUDA(cudaMemsetAsync(base, 0, xk::bicg_grid_bytes(x.n, nv), st));
+        double *hist = (double *)(base + goff[0]);
+        int *flags = (int *)(hist + GRID_ITERS * nv);
+        const xk::BicgGridArgs g{a.rpp(), a.cip(), a.val(prec), r0.p(), r.p(), x.p(), s.p(), t.p(),
+                                 {p.p(), base + goff[1]}, {v.p(), base + goff[2]}, base, hist, flags, flags + 1};
+        for (int it0 = 1;; it0 += GRID_ITERS) {
+            // the first iteration runs whatever max_iters says
+            const int it1 = (int)std::min<i64>((i64)it0 + GRID_ITERS, (i64)std::max(max_iters, 1) + 1);
+            XCUDA(cudaMemsetAsync(flags, 0, 2 * sizeof(int), st));
+            const cudaError_t e = xk::bicg_grid(prec, nv, g, x.n, it0, it1, sc, st);
+            if (e == cudaErrorCooperativeLaunchTooLarge && it0 == 1) {
+                cudaGetLastError();
+                return false;
+            }
+            XCUDA(e);
+            XCUDA(cudaMemcpyAsync(hhist.data(), hist, sizeof(double) * hhist.size(), cudaMemcpyDeviceToHost, st));
+            XCUDA(cudaStreamSynchronize(st));
+            int f[2];
+            std::memcpy(f, hhist.data() + GRID_ITERS * nv, sizeof f);
+            if (f[0]) throw Error("BiCGStab: a wait between the blocks of an iteration ran out");
+            for (int it = it0; it < it0 + f[1]; ++it) {
+                conv.iters = it;
+                conv.update(hhist.data() + (size_t)(it - it0) * nv);
+                conv.record();
+                if (conv.check() || it >= max_iters) return true;
+            }
+        }
     }
 
     // PCG (pcg.inl:48-160).  The step's two inner products (r,z), (p,Ap) are

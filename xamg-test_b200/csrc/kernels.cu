@@ -1601,6 +1601,481 @@ __device__ __forceinline__ void bicg_epi_col(int k, const double *val, const Bic
     }
 }
 
+// Whole BiCGStab iterations (no preconditioner) in one cooperative launch.  On
+// small systems the iteration above is eight launches of 2 to 5 us with little in
+// them, the gaps between, and a host read; here a CTA keeps its chunks of 256
+// rows (their matrix rows in shared memory, where they fit) and the grid meets
+// only where a product needs all rows: at the three inner products, whose chunk
+// partials are also the barrier.  A partial is published in two 64-bit words of
+// 32 value bits and the iteration's number each, after a fence behind the CTA's
+// vector stores (by a thread that has no partial to sum); every CTA polls all
+// partials of a column, one warp per column and pair, folds them in the tree of
+// k_dot2, and computes the scalar recurrences for itself.  FLY: the products form
+// s = r - alpha v and p = r + c1 v + beta p of the rows they gather as they go
+// (the owner stores its own for later), so neither needs a meeting of its own; p
+// and v are double-buffered for it.  Otherwise the owner stores them and the grid
+// meets again.  Vectors that change are read past L1 (other SMs write them).
+// Every expression and every sum is that of the separate kernels.
+// Bound: latency, about a third each of meetings (fence, store, poll, fold and
+// division: 2200 cycles with no other CTA to wait for), of products behind L2
+// gathers, and of waiting for the last CTA.
+// Measured (FP64, us per iteration, separate kernels -> this): 7-point 32^3 NV 1
+// 58.2 -> 13.8, NV 16 230 -> 41; 27-point 32^3 NV 1 70.2 -> 18.3; 27-point 40^3
+// NV 8 113 -> 58.
+struct BicgGridSlot {
+    unsigned long long lo, hi;
+};
+__device__ __forceinline__ void grid_fence() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ void slot_put(BicgGridSlot *q, double v, unsigned epoch) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v), e = (unsigned long long)epoch << 32;
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(q), "l"(e | (b & 0xffffffffull)), "l"(e | (b >> 32))
+                 : "memory");
+}
+__device__ __forceinline__ bool slot_get(const BicgGridSlot *q, unsigned epoch, double &v) {
+    unsigned long long a, b;
+    asm volatile("ld.acquire.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(q) : "memory");
+    v = __longlong_as_double((long long)((b << 32) | (a & 0xffffffffull)));
+    return (unsigned)(a >> 32) == epoch && (unsigned)(b >> 32) == epoch;
+}
+
+// The sum of one column's nch chunk partials (the k_dot2 tree), by one warp:
+// lane l holds the slots l, l + 32, ..., so the folds by 128, 64 and 32 are its own.
+__device__ __forceinline__ bool slots_sum(const BicgGridSlot *q, int nch, unsigned epoch, int *err, double &out) {
+    const int lane = threadIdx.x & 31;
+    double a[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) a[i] = 0.0;
+    bool ok = true;
+    for (int base = 0; base < nch; base += 256) {
+        double v[8];
+        unsigned pend = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (base + lane + 32 * i < nch) pend |= 1u << i;
+        const unsigned have = pend;
+        unsigned spins = 0;
+        unsigned long long t0 = 0;
+        while (pend) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+                if ((pend >> i) & 1u) {
+                    double w;
+                    if (slot_get(q + base + lane + 32 * i, epoch, w)) {
+                        v[i] = w;
+                        pend &= ~(1u << i);
+                    }
+                }
+            if ((++spins & 255) == 0) {
+                if (*(volatile int *)err) ok = false;
+                if (t0 == 0) t0 = gtime();
+                else if (gtime() - t0 > kWaitLimitNs) {
+                    atomicExch(err, 1);
+                    ok = false;
+                }
+                if (!ok) break;
+            }
+        }
+        if (!ok) break;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if ((have >> i) & 1u) a[i] = dadd(a[i], v[i]);
+    }
+    ok = __all_sync(0xffffffffu, ok);
+#pragma unroll
+    for (int off = 4; off >= 1; off >>= 1)
+#pragma unroll
+        for (int i = 0; i < off; ++i) a[i] = dadd(a[i], a[i + off]);
+    double v = a[0];
+#pragma unroll
+    for (int off = 16; off >= 1; off >>= 1) v = dadd(v, __shfl_xor_sync(0xffffffffu, v, off));
+    out = v;
+    return ok;
+}
+
+template <class T> struct BicgGrid {
+    const int *rp, *ci;
+    const T *va, *r0;
+    T *r, *x, *s, *t, *p[2], *v[2];
+    BicgGridSlot *slot;  // 5 NV nch partials (1, 3 and 1 pairs), then one word per CTA of the plain meetings
+    double *hist;        // residuals, NV per iteration of this launch
+    int *err, *done;     // error flag; iterations run
+};
+
+template <class T, int NV> struct BicgGridShape {
+    static constexpr int PK = 258;  // column stride of the chunk's operands (spreads a warp's rows over the banks)
+    static constexpr size_t SMEM = sizeof(T) * 2 * NV * PK;
+    static constexpr int NT = Shape<T, NV>::TPR == 1 ? 256 : 512;  // threads: a chunk's rows in few passes
+};
+
+// the V values at offset o (whose first column is k0) of a vector, and of s and
+// p formed from theirs (f, g: the columns' scalars)
+template <class T, int V> struct GridVec {
+    const T *x;
+    __device__ __forceinline__ void get(i64 o, T (&z)[V]) const { ld_cg<T, V>(x + o, z); }
+};
+template <class T, int V> struct GridS {
+    const T *r, *v;
+    const double *f;
+    __device__ __forceinline__ void get(i64 o, T (&z)[V]) const {
+        T a[V], b[V];
+        ld_cg<T, V>(r + o, a);
+        ld_cg<T, V>(v + o, b);
+#pragma unroll
+        for (int e = 0; e < V; ++e)
+            z[e] = (T)dadd(dmul(1.0, (double)a[e]), dmul(dmul(-1.0, f[e]), (double)b[e]));
+    }
+};
+template <class T, int V> struct GridP {
+    const T *p, *r, *v;
+    const double *f, *g;
+    bool first;  // p is r0 as it stands
+    __device__ __forceinline__ void get(i64 o, T (&z)[V]) const {
+        T a[V], b[V], c[V];
+        ld_cg<T, V>(p + o, c);
+        ld_cg<T, V>(r + o, a);
+        ld_cg<T, V>(v + o, b);
+#pragma unroll
+        for (int e = 0; e < V; ++e)
+            z[e] = first ? c[e]
+                         : (T)dadd(dadd(dmul(1.0, (double)a[e]), dmul(f[e], (double)b[e])), dmul(g[e], (double)c[e]));
+    }
+};
+// entries j0 .. j1 - 1 of one row of a product, GB entries and their gathers at a
+// time; the matrix from shared memory (SM) or global
+template <class T, int NV, int GB, bool SM, class X>
+__device__ __forceinline__ void grid_row(const int *__restrict__ ci, const T *__restrict__ va, int j0, int j1, int k0,
+                                         const X &x, T (&acc)[Shape<T, NV>::V]) {
+    constexpr int V = Shape<T, NV>::V;
+#pragma unroll
+    for (int e = 0; e < V; ++e) acc[e] = T(0);
+    for (int j = j0; j < j1; j += GB) {
+        int c[GB];
+        T v[GB], xv[GB][V];
+#pragma unroll
+        for (int k = 0; k < GB; ++k) {
+            const int u = min(j + k, j1 - 1);  // past the end: the last entry again, not added
+            c[k] = SM ? ci[u] : __ldg(ci + u);
+            v[k] = SM ? va[u] : __ldg(va + u);
+        }
+#pragma unroll
+        for (int k = 0; k < GB; ++k) x.get((i64)c[k] * NV + k0, xv[k]);
+#pragma unroll
+        for (int k = 0; k < GB; ++k)
+            if (j + k < j1)
+#pragma unroll
+                for (int e = 0; e < V; ++e) acc[e] = fma(v[k], xv[k][e], acc[e]);
+    }
+}
+
+template <class T, int NV, bool FLY>
+__global__ void __launch_bounds__(BicgGridShape<T, NV>::NT, BicgGridShape<T, NV>::NT == 256 ? 2 : 1) k_bicg_grid(BicgGrid<T> g, i64 n, int nch, int cpc, int ecap, int it0, int it1, BicgScalars sc) {
+    constexpr int V = Shape<T, NV>::V, TPR = Shape<T, NV>::TPR, NT = BicgGridShape<T, NV>::NT, RPB = NT / TPR, NP = 256 / RPB, PK = BicgGridShape<T, NV>::PK;
+    constexpr int GB = V * (FLY ? 3 : 1) * (int)sizeof(T) > 24 ? 4 : 8;
+    extern __shared__ __align__(16) unsigned char raw[];
+    T *sa = reinterpret_cast<T *>(raw), *sb = sa + NV * PK;
+    // the CTA's rows of the matrix, when they fit
+    T *sm_v = sb + NV * PK;
+    int *sm_c = reinterpret_cast<int *>(sm_v + ecap), *sm_r = sm_c + ecap;
+    __shared__ double val[3 * NV], rho[NV], alpha[NV], omega[NV], beta[NV], c1[NV], ac[NV], oc[NV], iconv[NV],
+        status[NV];
+    __shared__ int bad;
+    const int tid = threadIdx.x, warp = tid >> 5, wl = tid & 31, lane = tid % TPR, k0 = lane * V;
+    if (tid < NV) {
+        rho[tid] = sc.rho[tid];
+        beta[tid] = sc.beta[tid];
+        c1[tid] = sc.c1[tid];
+        iconv[tid] = sc.iconv[tid];
+        status[tid] = sc.status[tid];
+    }
+    if (tid == 0) bad = 0;
+    const int clo = blockIdx.x * cpc, chi = min(clo + cpc, nch);  // its chunks
+    const i64 lo = (i64)clo * 256, hi = (i64)chi * 256 < n ? (i64)chi * 256 : n;
+    const int e0 = __ldg(g.rp + lo), e1 = __ldg(g.rp + hi);
+    const bool kept = e1 - e0 <= ecap;
+    for (int q = tid; q <= (int)(hi - lo); q += NT) sm_r[q] = __ldg(g.rp + lo + q);
+    if (kept)
+        for (int j = tid; j < e1 - e0; j += NT) {
+            sm_v[j] = __ldg(g.va + e0 + j);
+            sm_c[j] = __ldg(g.ci + e0 + j);
+        }
+    __syncthreads();
+
+    // partials of this chunk's pairs (operands in sa, sb), one warp per pair and
+    // column, while the last warp waits until the CTA's stores are visible
+    auto publish = [&](int nd, int c, BicgGridSlot *slots, int it) {
+        __syncthreads();
+        if (tid == NT - 1) grid_fence();
+        for (int q = warp; q < nd * NV; q += NT / 32) {
+            const int d = q / NV, k = q % NV;
+            const T *A = (d == 2 ? sb : sa) + k * PK, *B = (nd == 3 && d == 1 ? sa : sb) + k * PK;
+            double acc = 0.0;
+#pragma unroll
+            for (int m = 0; m < 8; ++m)
+                if ((i64)c * 256 + 32 * m + wl < n) acc = fma((double)A[32 * m + wl], (double)B[32 * m + wl], acc);
+#pragma unroll
+            for (int off = 16; off >= 1; off >>= 1) acc = dadd(acc, __shfl_xor_sync(0xffffffffu, acc, off));
+            if (wl == 0) val[q] = acc;
+        }
+        __syncthreads();
+        if (tid < nd * NV) slot_put(slots + (i64)tid * nch + c, val[tid], (unsigned)it);
+    };
+    // the sums over all chunks into val; false: a wait ran out
+    auto collect = [&](int nd, const BicgGridSlot *slots, int it) {
+        for (int q = warp; q < nd * NV; q += NT / 32) {
+            double v;
+            const bool ok = slots_sum(slots + (i64)q * nch, nch, (unsigned)it, g.err, v);
+            if (wl == 0) {
+                val[q] = v;
+                if (!ok) bad = 1;
+            }
+        }
+        __syncthreads();
+        return bad == 0;
+    };
+    BicgGridSlot *const slotA = g.slot, *const slotB = slotA + (i64)NV * nch, *const slotC = slotB + (i64)3 * NV * nch,
+                 *const slotM = slotC + (i64)NV * nch;
+    auto meet = [&](unsigned epoch) {
+        __syncthreads();
+        if (warp == 0) {
+            if (wl == 0) {
+                grid_fence();
+                slot_put(slotM + blockIdx.x, 0.0, epoch);
+            }
+            double v;
+            const bool ok = slots_sum(slotM, (int)gridDim.x, epoch, g.err, v);
+            if (wl == 0 && !ok) bad = 1;
+        }
+        __syncthreads();
+        return bad == 0;
+    };
+#define GROW(...)                                                                                  \
+    {                                                                                              \
+        const int j0 = sm_r[row - lo], j1 = sm_r[row - lo + 1];                                    \
+        if (kept) grid_row<T, NV, GB, true>(sm_c, sm_v, j0 - e0, j1 - e0, k0, __VA_ARGS__, acc); \
+        else grid_row<T, NV, GB, false>(g.ci, g.va, j0, j1, k0, __VA_ARGS__, acc);                 \
+    }
+    int it = it0;
+    for (; it < it1; ++it) {
+        T *const pn = g.p[FLY ? it & 1 : 0], *const vn = g.v[FLY ? it & 1 : 0];
+        const T *const po = g.p[FLY ? (it & 1) ^ 1 : 0], *const vo = g.v[FLY ? (it & 1) ^ 1 : 0];
+        const GridP<T, V> gp{po, g.r, vo, c1 + k0, beta + k0, it == 1};
+        if (!FLY && it > 1) {
+            for (int c = clo; c < chi; ++c)
+                for (int h = 0; h < NP; ++h) {
+                    const i64 row = (i64)c * 256 + h * RPB + tid / TPR;
+                    if (row >= n) continue;
+                    T z[V];
+                    gp.get(row * NV + k0, z);
+                    st<T, V>(pn + row * NV + k0, z);
+                }
+            if (!meet(2u * (unsigned)it)) return;
+        }
+        // v = A p, (v, r0)
+        for (int c = clo; c < chi; ++c) {
+            for (int h = 0; h < NP; ++h) {
+                const int q = h * RPB + tid / TPR;
+                const i64 row = (i64)c * 256 + q;
+                if (row >= n) continue;
+                const i64 o = row * NV + k0;
+                T acc[V], z[V];
+                if (FLY) {
+                    gp.get(o, z);
+                    st<T, V>(pn + o, z);
+                    GROW(gp);
+                } else {
+                    GROW(GridVec<T, V>{pn});
+                }
+                ld<T, V>(g.r0 + o, z);
+                st<T, V>(vn + o, acc);
+#pragma unroll
+                for (int e = 0; e < V; ++e) {
+                    sa[(k0 + e) * PK + q] = acc[e];
+                    sb[(k0 + e) * PK + q] = z[e];
+                }
+            }
+            publish(1, c, slotA, it);
+        }
+        if (!collect(1, slotA, it)) return;
+        if (tid < NV) alpha[tid] = __ddiv_rn(rho[tid], val[tid]);
+        __syncthreads();
+
+        // s = r - alpha v, t = A s, (t, s), (t, t), (s, s)
+        const GridS<T, V> gs{g.r, vn, alpha + k0};
+        if (!FLY) {
+            for (int c = clo; c < chi; ++c)
+                for (int h = 0; h < NP; ++h) {
+                    const i64 row = (i64)c * 256 + h * RPB + tid / TPR;
+                    if (row >= n) continue;
+                    T z[V];
+                    gs.get(row * NV + k0, z);
+                    st<T, V>(g.s + row * NV + k0, z);
+                }
+            if (!meet(2u * (unsigned)it + 1u)) return;
+        }
+        for (int c = clo; c < chi; ++c) {
+            for (int h = 0; h < NP; ++h) {
+                const int q = h * RPB + tid / TPR;
+                const i64 row = (i64)c * 256 + q;
+                if (row >= n) continue;
+                const i64 o = row * NV + k0;
+                T acc[V], z[V];
+                if (FLY) {
+                    gs.get(o, z);
+                    st<T, V>(g.s + o, z);
+                    GROW(gs);
+                } else {
+                    ld_cg<T, V>(g.s + o, z);
+                    GROW(GridVec<T, V>{g.s});
+                }
+                st<T, V>(g.t + o, acc);
+#pragma unroll
+                for (int e = 0; e < V; ++e) {
+                    sa[(k0 + e) * PK + q] = acc[e];
+                    sb[(k0 + e) * PK + q] = z[e];
+                }
+            }
+            publish(3, c, slotB, it);
+        }
+        // the first rows' operands of the next pass are the thread's own: read ahead
+        T pa[V], ps[V], px[V], pt[V];
+        const i64 prow = (i64)clo * 256 + tid / TPR, po1 = (prow < n ? prow : 0) * NV + k0;
+        ld_cg<T, V>(pn + po1, pa);
+        ld_cg<T, V>(g.s + po1, ps);
+        ld_cg<T, V>(g.x + po1, px);
+        ld_cg<T, V>(g.t + po1, pt);
+        if (!collect(3, slotB, it)) return;
+        if (tid < NV) {  // bicg_epi_col<EPI_OMEGA>
+            const double s2 = val[tid], s3 = val[NV + tid], s4 = val[2 * NV + tid], w = __ddiv_rn(s2, s3), ic = iconv[tid];
+            omega[tid] = w;
+            ac[tid] = dmul(ic, alpha[tid]);
+            oc[tid] = dmul(ic, w);
+            const double rs = dadd(dmul(1.0, s4), dmul(-1.0, dmul(w, s2)));
+            if (blockIdx.x == 0) g.hist[(i64)(it - it0) * NV + tid] = rs;
+            if (sc.check && status[tid] == 0.0 && !(__dsqrt_rn(rs) > sc.tol[tid])) status[tid] = 1.0;
+            iconv[tid] = status[tid] != 0.0 ? 0.0 : 1.0;
+        }
+        __syncthreads();
+        bool stop = sc.check != 0;
+        for (int k = 0; k < NV; ++k) stop = stop && status[k] != 0.0;
+
+        // x += ac p + oc s, r = s - omega t, (r, r0)
+        for (int c = clo; c < chi; ++c) {
+            for (int h = 0; h < NP; ++h) {
+                const int q = h * RPB + tid / TPR;
+                const i64 row = (i64)c * 256 + q;
+                if (row >= n) continue;
+                const i64 o = row * NV + k0;
+                T a[V], xx[V], sv[V], tv[V], z[V];
+                ld<T, V>(g.r0 + o, z);
+                if (c == clo && h == 0) {
+#pragma unroll
+                    for (int e = 0; e < V; ++e) {
+                        a[e] = pa[e];
+                        sv[e] = ps[e];
+                        xx[e] = px[e];
+                        tv[e] = pt[e];
+                    }
+                } else {
+                    ld_cg<T, V>(pn + o, a);
+                    ld_cg<T, V>(g.s + o, sv);
+                    ld_cg<T, V>(g.x + o, xx);
+                    ld_cg<T, V>(g.t + o, tv);
+                }
+#pragma unroll
+                for (int e = 0; e < V; ++e) {
+                    const int k = k0 + e;
+                    xx[e] = (T)dadd(dadd(dmul(ac[k], (double)a[e]), dmul(oc[k], (double)sv[e])),
+                                    dmul(1.0, (double)xx[e]));
+                    tv[e] = (T)dadd(dmul(1.0, (double)sv[e]), dmul(dmul(-1.0, omega[k]), (double)tv[e]));
+                    sa[k * PK + q] = tv[e];
+                    sb[k * PK + q] = z[e];
+                }
+                st<T, V>(g.x + o, xx);
+                st<T, V>(g.r + o, tv);
+            }
+            if (!stop) publish(1, c, slotC, it);
+        }
+        if (stop) {
+            ++it;
+            break;
+        }
+        if (!collect(1, slotC, it)) return;
+        if (tid < NV) {  // bicg_epi_col<EPI_BETA>
+            const double s1 = val[tid], bt = dmul(__ddiv_rn(s1, rho[tid]), __ddiv_rn(alpha[tid], omega[tid]));
+            beta[tid] = bt;
+            rho[tid] = s1;
+            c1[tid] = dmul(-1.0, dmul(omega[tid], bt));
+        }
+        __syncthreads();
+    }
+    if (blockIdx.x == 0) {
+        if (tid < NV) {  // for a launch that goes on from here
+            sc.rho[tid] = rho[tid];
+            sc.beta[tid] = beta[tid];
+            sc.c1[tid] = c1[tid];
+            sc.iconv[tid] = iconv[tid];
+            sc.status[tid] = status[tid];
+        }
+        if (tid == 0) *g.done = it - it0;
+    }
+#undef GROW
+}
+
+size_t bicg_grid_bytes(i64 n, int nv) {
+    const i64 nch = (n + 255) / 256;
+    return sizeof(BicgGridSlot) * (size_t)(5 * nv * nch + nch);
+}
+
+template <class T, int NV, bool FLY>
+static cudaError_t bicg_grid_l(const BicgGridArgs &a, i64 n, int it0, int it1, const BicgScalars &sc, cudaStream_t s) {
+    auto k = k_bicg_grid<T, NV, FLY>;
+    constexpr int NT = BicgGridShape<T, NV>::NT;
+    // two CTAs of 256 threads on an SM when there are chunks for them
+    int nch = (int)((n + 255) / 256);
+    const int per = NT == 256 && nch > sm_count() ? 2 : 1, slots = per * sm_count();
+    int cpc = (nch + slots - 1) / slots;
+    const size_t room = (size_t)(per == 1 ? 220 : 110) * 1024, base = BicgGridShape<T, NV>::SMEM;
+    const size_t rows = sizeof(int) * ((size_t)cpc * 256 + 1);
+    int ecap = room > base + rows ? (int)((room - base - rows) / (sizeof(T) + 4)) / 2 * 2 : 0;
+    const size_t smem = base + rows + (size_t)ecap * (sizeof(T) + 4);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    BicgGrid<T> g{a.rp, a.ci, (const T *)a.va, (const T *)a.r0, (T *)a.r, (T *)a.x, (T *)a.s, (T *)a.t,
+                  {(T *)a.p[0], (T *)a.p[1]}, {(T *)a.v[0], (T *)a.v[1]}, (BicgGridSlot *)a.slots, a.hist, a.err, a.done};
+    BicgScalars scv = sc;
+    void *args[] = {&g, &n, &nch, &cpc, &ecap, &it0, &it1, &scv};
+    note_launch();
+    return cudaLaunchCooperativeKernel((const void *)k, dim3((unsigned)((nch + cpc - 1) / cpc)), dim3(NT), args, smem, s);
+}
+
+// Gathering two or three vectors for each entry against one more meeting: up to
+// 32 bytes per row it wins (us per iteration with and without, FP64 32^3: 7-point
+// NV 1 14.8 and 22.1, NV 4 19.2 and 24.0; 27-point NV 4 27.4 and 29.8), beyond it
+// loses (27-point NV 8 42.9 and 39.2, NV 16 66.0 and 54.6).
+template <class T, int NV> constexpr bool bicg_fly_v = NV * sizeof(T) <= 32;
+bool bicg_grid_fly(Prec p, int nv) { return nv * (p == Prec::F64 ? 8 : 4) <= 32; }
+
+// Two chunks per SM: at 40^3 (250 chunks) every operator and width gains (7-point
+// NV 1 57.9 -> 19.1 us per iteration, 27-point NV 16 247 -> 101), at 64^3 the
+// separate kernels have work enough (7-point NV 1 62 -> 53, NV 8 157 -> 139, but
+// 27-point NV 1 133 -> 271, its matrix no longer in shared memory).
+bool bicg_grid_fits(i64 n) { return n > 0 && (n + 255) / 256 <= 2 * sm_count(); }
+
+cudaError_t bicg_grid(Prec p, int nv, const BicgGridArgs &a, i64 n, int it0, int it1, const BicgScalars &sc,
+                      cudaStream_t s) {
+    cudaError_t e = cudaErrorInvalidValue;
+    if (p == Prec::F64) {
+#define F(NV) e = bicg_grid_l<double, NV, bicg_fly_v<double, NV>>(a, n, it0, it1, sc, s)
+        NV_DISPATCH(nv, F)
+#undef F
+    } else {
+#define F(NV) e = bicg_grid_l<float, NV, bicg_fly_v<float, NV>>(a, n, it0, it1, sc, s)
+        NV_DISPATCH(nv, F)
+#undef F
+    }
+    return e;
+}
+
 template <class T, int NV>
 static void bicg_groups_t(int grp, i64 n, const BicgScalars &sc, const void *a0, const void *a1, void *a2,
                           const void *a3, const void *a4, void *a5, const void *a6, double *part, cudaStream_t s) {

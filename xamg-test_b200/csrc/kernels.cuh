@@ -193,6 +193,25 @@ struct BicgScalars {
     double *rho, *alpha, *omega, *beta, *c1, *ac, *oc, *res, *iconv, *status, *tol;
     int check;  // 1: update status/iconv from res and tol in the omega stage
 };
+// Iterations it0 .. it1 - 1 (counted from 1) of BiCGStab without a
+// preconditioner in one cooperative launch, stopping after the one at which all
+// columns have converged (sc.check); the same bits as the separate kernels.
+// slots: bicg_grid_bytes, zeroed before iteration 1; hist: NV residuals per
+// iteration of the launch; done: iterations run; err: set when a wait ran out.
+// For systems that bicg_grid_fits.  p[1], v[1]: second buffers, needed where bicg_grid_fly (p[0] holds the first
+// direction, p and v of either buffer the last ones afterwards).
+struct BicgGridArgs {
+    const int *rp, *ci;
+    const void *va, *r0;
+    void *r, *x, *s, *t, *p[2], *v[2], *slots;
+    double *hist;
+    int *err, *done;
+};
+bool bicg_grid_fits(i64 n);
+bool bicg_grid_fly(Prec p, int nv);
+size_t bicg_grid_bytes(i64 n, int nv);
+cudaError_t bicg_grid(Prec p, int nv, const BicgGridArgs &a, i64 n, int it0, int it1, const BicgScalars &sc,
+                      cudaStream_t s);
 // first stage of dots() alone: chunk partials of nd pairs into part
 void dot_partials(Prec in, int nv, i64 n, int nd, const void *const *a, const void *const *b, double *part,
                   cudaStream_t s);
