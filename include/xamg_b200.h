@@ -199,8 +199,9 @@ int xamg_csr_spmv(int prec, int nv, int64_t n, const int *rp, const int *ci, con
  * 0, 1, 2 = one CTA per row tile with x gathers issued 4, 8 or 16 entries at
  * a time; 3, 4 = the tile's entries staged in shared memory, gathers 4 or 8 at
  * a time; 5, 6 = staged entries with a plain row loop unrolled 4 or 8 times;
- * 10 + k = staged streaming kernel walking k tiles per CTA; -1 = default (6
- * when nv * element size >= 64 bytes, else 0).  Under -1 and 7 the products
+ * 8 = a warp's rows side by side with their entries staged a step ahead;
+ * 10 + k = staged streaming kernel walking k tiles per CTA; -1 = default (by
+ * row width, and for the library's own operators by rows and entries).  Under -1 and 7 the products
  * of operators that have a shifted-row run plan (below) use the run kernel
  * (7 elsewhere = the default).  The setting belongs to the calling host
  * thread; a batch's autotuned choices are held by its own operators and are

@@ -104,7 +104,7 @@ void Batch::create(int nsys, const i64 *n, const int *const *rp, const int *cons
 void Batch::autotune(BatchGroup &G) {
     cudaStream_t st = ctx().stream;
     const DCsr &a = G.A.d;
-    const int vars[] = {0, 1, 2, 3, 5, 6, 7};  // 7: shifted-row runs where the operator has a plan
+    const int vars[] = {0, 1, 2, 3, 5, 6, 7, 8};  // 7: shifted-row runs where the operator has a plan
     cudaEvent_t e0, e1;
     XCUDA(cudaEventCreate(&e0));
     XCUDA(cudaEventCreate(&e1));

@@ -174,7 +174,7 @@ void DCsr::spmv(Prec p, int nv, const void *x, void *y, int mode, const void *b,
         return;
     }
     KTimeScope kt(KClass::SPMV, n, (double)nnz * (sv + 4) + (double)(n + 1) * 4 + xy, s);
-    xk::spmv(p, nv, n, rpp(), cip(), val(p), x, y, mode, b, s, var);
+    xk::spmv(p, nv, n, rpp(), cip(), val(p), x, y, mode, b, s, var, nnz);
 }
 
 }  // namespace xamg

@@ -304,9 +304,107 @@ __global__ void __launch_bounds__(256, LOOP == 1 ? 6 : 1) k_spmv_tile(i64 n, con
     st<T, V>(y + row * NV + lane * V, acc);
 }
 
+// Rows side by side: a warp's RPW rows advance together, KS entries a step.  The
+// entries of the next step are copied into shared memory (cp.async; the lanes
+// that copy a row's entries are neighbours, so the copies coalesce) while this
+// step's x gathers, eight under way per row, feed the chains.  Read row by row from
+// global memory, every column and value would take an L1 wavefront of its own
+// beside the gather's; staged tile by tile, rows wait for the longest of theirs
+// chunk after chunk.  Same per-row summation order as k_spmv.
+// Bound: L1 wavefronts of the gathers; on small operators the latency of a
+// step (irregular 4000 rows of 41 entries, FP32 NV 16: 7.7 us, tile-staged 16.9).
+// Eight entries a step where 16 cost registers or shared memory (FP64 NV 8, the
+// same operator: 9.1 us against 14.1).
+template <class T, int NV> struct RowsShape {
+    static constexpr int TPR = Shape<T, NV>::TPR, RPW = 32 / TPR, KS = TPR == 1 || (TPR == 4 && sizeof(T) == 8) ? 8 : 16, NW = 4;
+    static constexpr int SLOTS = RPW * KS, CP = (SLOTS + 31) / 32, PAD = KS + 1;
+};
+__device__ __forceinline__ void cp_async_elem(int *dst, const int *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_elem(float *dst, const float *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_elem(double *dst, const double *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+template <class T, int NV, int MODE>
+__global__ void __launch_bounds__(128) k_spmv_rows(i64 n, const int *__restrict__ rp, const int *__restrict__ ci,
+                                                   const T *__restrict__ va, const T *__restrict__ x,
+                                                   T *__restrict__ y, const T *__restrict__ b) {
+    typedef RowsShape<T, NV> S;
+    constexpr int V = Shape<T, NV>::V, TPR = S::TPR, RPW = S::RPW, KS = S::KS, GB = 8;
+    __shared__ int s_c[S::NW][2][RPW * S::PAD];
+    __shared__ T s_v[S::NW][2][RPW * S::PAD];
+    const int warp = threadIdx.x >> 5, wl = threadIdx.x & 31, lane = wl % TPR, q = wl / TPR;
+    const i64 r0 = ((i64)blockIdx.x * S::NW + warp) * RPW, row = r0 + q;
+    if (r0 >= n) return;
+    const bool live = row < n;
+    const int j0 = __ldg(rp + min(row, n)), j1 = __ldg(rp + min(row + 1, n));
+    const int steps = (__reduce_max_sync(0xffffffffu, j1 - j0) + KS - 1) / KS;
+    // the slots this lane copies: row (wl + 32 i) / KS, entry (wl + 32 i) % KS of a step
+    int cj[S::CP], ce[S::CP];
+#pragma unroll
+    for (int i = 0; i < S::CP; ++i) {
+        const int sl = wl + 32 * i, rq = sl / KS;
+        cj[i] = __shfl_sync(0xffffffffu, j0, (rq * TPR) & 31) + sl % KS;
+        ce[i] = __shfl_sync(0xffffffffu, j1, (rq * TPR) & 31);
+        if (sl >= S::SLOTS) ce[i] = 0;
+    }
+    auto stage = [&](int st) {
+        int *sc = s_c[warp][st & 1];
+        T *sv = s_v[warp][st & 1];
+#pragma unroll
+        for (int i = 0; i < S::CP; ++i) {
+            const int sl = wl + 32 * i, o = sl / KS * S::PAD + sl % KS, j = cj[i] + st * KS;
+            if (j < ce[i]) {
+                cp_async_elem(sc + o, ci + j);
+                cp_async_elem(sv + o, va + j);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    T acc[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) acc[e] = T(0);
+    const T *xb = x + lane * V;
+    stage(0);
+    if (MODE == 1 && live) ld<T, V>(y + row * NV + lane * V, acc);
+    for (int st = 0; st < steps; ++st) {
+        stage(st + 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        const int *sc = s_c[warp][st & 1] + q * S::PAD;
+        const T *sv = s_v[warp][st & 1] + q * S::PAD;
+        const int m = min(KS, j1 - j0 - st * KS);
+#pragma unroll
+        for (int k0 = 0; k0 < KS; k0 += GB) {
+            T xv[GB][V];
+#pragma unroll
+            for (int k = 0; k < GB; ++k)
+                if (k0 + k < m) ld<T, V>(xb + (i64)sc[k0 + k] * NV, xv[k]);
+#pragma unroll
+            for (int k = 0; k < GB; ++k)
+                if (k0 + k < m)
+#pragma unroll
+                    for (int e = 0; e < V; ++e) acc[e] = fma(sv[k0 + k], xv[k][e], acc[e]);
+        }
+        __syncwarp();
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if (!live) return;
+    if (MODE == 2) {
+        T bb[V];
+        ld<T, V>(b + row * NV + lane * V, bb);
+#pragma unroll
+        for (int e = 0; e < V; ++e) acc[e] = add_rn<T>(mul_rn<T>(T(1), bb[e]), mul_rn<T>(T(-1), acc[e]));
+    }
+    st<T, V>(y + row * NV + lane * V, acc);
+}
+
 // SpMV variant selection: 0, 1, 2 = row kernel with gather batches of 4, 8,
 // 16 entries; 3, 4 = tile-staged kernel with batches of 4, 8; 5, 6 = the same
-// with a plain row loop unrolled 4, 8 times; 10 + k = streaming kernel
+// with a plain row loop unrolled 4, 8 times; 8 = rows side by side; 10 + k = streaming kernel
 // walking k tiles per CTA; -1 = default (6 when NV*sizeof(T) >= 64 bytes,
 // else 0).
 static thread_local int g_spmv_variant = -1;
@@ -332,17 +430,48 @@ static int sm_count() {
     return sms;
 }
 
+// The kernel of a product with n rows and nnz entries (-1: not known).  Measured
+// (us, k_spmv_rows / k_spmv GB 4 / GB 8 / k_spmv_tile):
+//   rows of 16 entries and more, any width: the rows side by side (irregular
+//   4000 rows of 41, FP64 NV 4 8.3 / 13.5 / 16.2 / 17.8; FP32 NV 16 7.7 / 12.6 /
+//   12.8 / 16.9; 27-point 24^3 FP32 NV 8 3.9 / 4.7 / 4.9 / 6.0), but
+//   wide rows of less than 32, many of them: tile-staged (27-point 64^3 FP32 NV 16
+//   47 / 41 / 44 / 34; 24^3 4.1 / 4.8 / 5.1 / 5.0), and
+//   FP64 NV 1, many rows: GB 8 (27-point 40^3 7.7 / 8.9 / 7.3 / 11.3, irregular
+//   55799 rows 24 / 27 / 21 / 32; 4000 rows 11.1 / 17.3 / 11.3 / 15.1);
+//   shorter rows: GB 4 (7-point 113x97x101 FP32 NV 8 60 / 33 / 43 / 45, FP64 NV 16
+//   157 / 150 / 166 / 154), in FP64 with one thread a row GB 8 (NV 1 32 / 23 / 21 / 26);
+//   not known: as for short rows, wide ones tile-staged (27-point 100^3 FP64 NV 16
+//   331 against 222, 7-point 150 against 154).
+template <class T, int NV>
+static int default_variant(i64 n, i64 nnz) {
+    constexpr int TPR = Shape<T, NV>::TPR;
+    constexpr bool f64 = sizeof(T) == 8;
+    if (nnz >= 16 * n) {
+        if (f64 && NV == 1) return n <= 32768 ? 8 : 1;
+        return TPR <= 2 || nnz >= 32 * n || n <= 20000 ? 8 : 6;
+    }
+    if (TPR == 1) return f64 ? 1 : 0;
+    return TPR >= 4 && nnz < 0 ? 6 : 0;
+}
+
 template <class T, int NV>
 static void spmv_t(i64 n, const int *rp, const int *ci, const T *va, const T *x, T *y, int mode,
-                   const T *b, cudaStream_t s, int choice) {
+                   const T *b, cudaStream_t s, int choice, i64 nnz) {
     constexpr int RPB = 256 / Shape<T, NV>::TPR;
     if (n <= 0) return;
     note_launch();
     i64 ntiles = (n + RPB - 1) / RPB;
-    // default: the tile-staged kernel when a row spans at least 4 threads (its
-    // tile of RPB rows then fits the shared-memory stage), else batches of 4
     const int want = choice >= 0 ? choice : g_spmv_variant;
-    int var = (want >= 0 && want != 7) ? want : (Shape<T, NV>::TPR >= 4 ? 6 : 0);
+    int var = (want >= 0 && want != 7) ? want : default_variant<T, NV>(n, nnz);
+    if (var == 8) {
+        constexpr int RPC = RowsShape<T, NV>::RPW * RowsShape<T, NV>::NW;
+        const unsigned g = (unsigned)((n + RPC - 1) / RPC);
+        if (mode == 0) k_spmv_rows<T, NV, 0><<<g, 128, 0, s>>>(n, rp, ci, va, x, y, b);
+        else if (mode == 1) k_spmv_rows<T, NV, 1><<<g, 128, 0, s>>>(n, rp, ci, va, x, y, b);
+        else k_spmv_rows<T, NV, 2><<<g, 128, 0, s>>>(n, rp, ci, va, x, y, b);
+        return;
+    }
     if (var >= 3 && var <= 6) {
         unsigned g = (unsigned)ntiles;
 #define L(GB, LOOP)                                                                                \
@@ -371,13 +500,13 @@ static void spmv_t(i64 n, const int *rp, const int *ci, const T *va, const T *x,
 }
 
 void spmv(Prec p, int nv, i64 n, const int *rp, const int *ci, const void *val, const void *x,
-          void *y, int mode, const void *b, cudaStream_t s, int variant) {
+          void *y, int mode, const void *b, cudaStream_t s, int variant, i64 nnz) {
     if (p == Prec::F64) {
-#define F(NV) spmv_t<double, NV>(n, rp, ci, (const double *)val, (const double *)x, (double *)y, mode, (const double *)b, s, variant)
+#define F(NV) spmv_t<double, NV>(n, rp, ci, (const double *)val, (const double *)x, (double *)y, mode, (const double *)b, s, variant, nnz)
         NV_DISPATCH(nv, F)
 #undef F
     } else {
-#define F(NV) spmv_t<float, NV>(n, rp, ci, (const float *)val, (const float *)x, (float *)y, mode, (const float *)b, s, variant)
+#define F(NV) spmv_t<float, NV>(n, rp, ci, (const float *)val, (const float *)x, (float *)y, mode, (const float *)b, s, variant, nnz)
         NV_DISPATCH(nv, F)
 #undef F
     }
