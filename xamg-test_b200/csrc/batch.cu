@@ -2,6 +2,7 @@
 // one block-diagonal system whose row segments carry their own Krylov scalars
 // (sm_100a).  Per-(segment, column) scalars live at [s*nv + k]; the vectors
 // are FP64 block vectors (row-major n x nv) of the concatenated systems.
+#include "dots.cuh"
 #include "kernels.cuh"
 #include <cuda_runtime.h>
 
@@ -23,49 +24,38 @@ __device__ __forceinline__ int seg_of(const i64 *segoff, int nseg, i64 i) {
     return lo;
 }
 
-// Stage 1 of the per-segment canonical inner products: one warp per chunk of
-// 256 rows of one segment (chunks counted from the segment's first row), the
-// same lane/row assignment and butterfly as the whole-vector dots.
-template <class TI, int NV, int ND>
-__global__ void __launch_bounds__(256) k_segdot1(int nseg, const i64 *__restrict__ segoff,
-                                                 const i64 *__restrict__ cstart, i64 nch,
+// Stage 1 of the per-segment canonical inner products: chunks of 256 rows of
+// one segment (counted from the segment's first row), in the order and with the
+// split of the whole-vector dots (dots.cuh).
+template <class TI, int NV, int ND, bool SH>
+__global__ void __launch_bounds__(256, ND == 1 ? 4 : 2) k_segdot1(int nseg, const i64 *__restrict__ segoff,
+                                                 const i64 *__restrict__ cstart, i64 nch, int W,
                                                  const TI *__restrict__ a0, const TI *__restrict__ b0,
                                                  const TI *__restrict__ a1, const TI *__restrict__ b1,
                                                  const TI *__restrict__ a2, const TI *__restrict__ b2,
                                                  double *__restrict__ part) {
+    constexpr int V = DotShape<NV>::V, C = ND * V;
+    __shared__ double sm[8 * C * 32];
     const int lane = threadIdx.x & 31;
-    const i64 g = (i64)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (g >= nch) return;
-    const int s = seg_of(cstart, nseg, g);
-    const i64 c = g - cstart[s];
-    const i64 r0 = segoff[s], r1 = segoff[s + 1];
-    const TI *A[3] = {a0, a1, a2};
-    const TI *B[3] = {b0, b1, b2};
-    double acc[ND][NV];
+    const i64 w = (i64)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), g = w / W;
+    const int sub = (int)(w % W);
+    const TI *const pa[3] = {a0, a1, a2}, *const pb[3] = {b0, b1, b2};
+    const TI *A[ND], *B[ND];
 #pragma unroll
-    for (int d = 0; d < ND; ++d)
-#pragma unroll
-        for (int k = 0; k < NV; ++k) acc[d][k] = 0.0;
-#pragma unroll 1
-    for (int m = 0; m < 8; ++m) {
-        const i64 i = r0 + c * 256 + 32 * m + lane;
-        if (i < r1) {
-#pragma unroll
-            for (int d = 0; d < ND; ++d)
-#pragma unroll
-                for (int k = 0; k < NV; ++k)
-                    acc[d][k] = fma((double)A[d][i * NV + k], (double)B[d][i * NV + k], acc[d][k]);
-        }
+    for (int d = 0; d < ND; ++d) { A[d] = pa[d]; B[d] = pb[d]; }
+    double v[C];
+    if (g < nch) {
+        const int s = seg_of(cstart, nseg, g);
+        const i64 r0 = segoff[s] + (g - cstart[s]) * 256;
+        dot_chunk<TI, NV, ND, SH>(A, B, r0, (int)min((i64)256, segoff[s + 1] - r0), W, sub, v);
     }
+    if (!dot_join<NV>(W, sub, sm, v) || g >= nch) return;
+    dot_fold_lanes<NV>(v);
+    if (lane < DotShape<NV>::TPR)
 #pragma unroll
-    for (int d = 0; d < ND; ++d)
+        for (int d = 0; d < ND; ++d)
 #pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            double v = acc[d][k];
-#pragma unroll
-            for (int off = 16; off >= 1; off >>= 1) v = dadd_(v, __shfl_xor_sync(0xffffffffu, v, off));
-            if (lane == 0) part[((i64)d * NV + k) * nch + g] = v;
-        }
+            for (int e = 0; e < V; ++e) part[((i64)d * NV + lane * V + e) * nch + g] = v[d * V + e];
 }
 
 // Stage 2: block (segment s, dot d, column k) folds the segment's chunks with
@@ -81,12 +71,16 @@ __global__ void __launch_bounds__(256) k_segdot2(int nseg, int ndk, int nv, cons
     for (i64 c = threadIdx.x; c < cn; c += 256) a = dadd_(a, p[c]);
     q[threadIdx.x] = a;
     __syncthreads();
-    for (int off = 128; off >= 32; off >>= 1) {
-        if (threadIdx.x < off) q[threadIdx.x] = dadd_(q[threadIdx.x], q[threadIdx.x + off]);
-        __syncthreads();
-    }
     if (threadIdx.x < 32) {
-        double v = q[threadIdx.x];
+        // the folds by 128, 64 and 32 are of this lane's own slots
+        double u[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) u[i] = q[threadIdx.x + 32 * i];
+#pragma unroll
+        for (int off = 4; off >= 1; off >>= 1)
+#pragma unroll
+            for (int i = 0; i < off; ++i) u[i] = dadd_(u[i], u[i + off]);
+        double v = u[0];
         for (int off = 16; off >= 1; off >>= 1) v = dadd_(v, __shfl_xor_sync(0xffffffffu, v, off));
         if (threadIdx.x == 0) {
             const int d = dk / nv, k = dk % nv;
@@ -180,13 +174,19 @@ static void segdots_t(int nseg, const i64 *segoff, const i64 *cstart, i64 nch, i
                       cudaStream_t s) {
     note_launch(nch > 0 ? 2 : 1);
     if (nch > 0) {
-        const unsigned g = (unsigned)((nch + 7) / 8);
         const TI *A0 = (const TI *)a[0], *B0 = (const TI *)b[0];
         const TI *A1 = nd > 1 ? (const TI *)a[1] : A0, *B1 = nd > 1 ? (const TI *)b[1] : B0;
         const TI *A2 = nd > 2 ? (const TI *)a[2] : A0, *B2 = nd > 2 ? (const TI *)b[2] : B0;
-        if (nd == 1) k_segdot1<TI, NV, 1><<<g, 256, 0, s>>>(nseg, segoff, cstart, nch, A0, B0, A1, B1, A2, B2, part);
-        else if (nd == 2) k_segdot1<TI, NV, 2><<<g, 256, 0, s>>>(nseg, segoff, cstart, nch, A0, B0, A1, B1, A2, B2, part);
-        else k_segdot1<TI, NV, 3><<<g, 256, 0, s>>>(nseg, segoff, cstart, nch, A0, B0, A1, B1, A2, B2, part);
+        const DotSplit sp = dot_split<NV>(nch, sm_count());
+        const bool sh = nd == 3 && A1 == A0 && B1 == A0 && A2 == B0 && B2 == B0;
+#define L(ND, SH)                                                                                   \
+    k_segdot1<TI, NV, ND, SH><<<sp.blocks, 32 * sp.warps, 0, s>>>(nseg, segoff, cstart, nch, sp.W, A0, B0, A1, B1, A2, \
+                                                                  B2, part)
+        if (nd == 1) L(1, false);
+        else if (nd == 2) L(2, false);
+        else if (sh) L(3, true);
+        else L(3, false);
+#undef L
     }
     k_segdot2<<<(unsigned)(nseg * nd * NV), 256, 0, s>>>(nseg, nd * NV, NV, cstart, nch, part, out);
 }

@@ -11,6 +11,7 @@
 //  * Row sums keep the stored CSR order (a sequential fma chain per (row,col)),
 //    which makes the result independent of the launch shape and bit-identical
 //    to the oracle.
+#include "dots.cuh"
 #include "kernels.cuh"
 #include <cooperative_groups.h>
 #include <atomic>
@@ -419,7 +420,7 @@ void note_launch(int k) { g_launches.fetch_add(k, std::memory_order_relaxed); }
 long long launch_count() { return g_launches.load(std::memory_order_relaxed); }
 int get_spmv_variant() { return g_spmv_variant; }
 
-static int sm_count() {
+int sm_count() {
     static int sms = 0;
     if (!sms) {
         int dev = 0;
@@ -1160,78 +1161,71 @@ void dense_gemv(Prec p, int nv, int n, const void *AinvT, const void *b, void *y
 }
 
 // ---------------------------------------------------------------- dots
-// Stage 1: one warp per 256-row chunk; lane l accumulates rows l, l+32, ...,
-// l+224 (fma, FP64), then a xor-butterfly over the 32 lanes (off = 16..1),
-// whose lane-0 value equals the pairwise tree s[l] += s[l+off].
-// Partials are stored dot-major: part[(d*nv + k) * nchunks + c].
+// Stage 1: a warp, or W of them, per 256-row chunk (dots.cuh has the order and
+// the split).  Partials are stored dot-major: part[(d*nv + k) * nchunks + c].
 template <class TI>
 struct DotPairs {
     const TI *a[4];
     const TI *b[4];
 };
-template <class TI, int NV, int ND>
-__global__ void __launch_bounds__(256) k_dot1(i64 n, i64 nch, DotPairs<TI> pr, double *__restrict__ part) {
+template <class TI, int NV, int ND, bool SH>
+__global__ void __launch_bounds__(256, ND == 1 ? 4 : 2) k_dot1(i64 n, i64 nch, int W, DotPairs<TI> pr, double *__restrict__ part) {
+    constexpr int V = DotShape<NV>::V, C = ND * V;
+    __shared__ double sm[8 * C * 32];
     const int lane = threadIdx.x & 31;
-    const i64 c = (i64)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (c >= nch) return;
-    const TI *__restrict__ A[ND];
-    const TI *__restrict__ B[ND];
+    const i64 w = (i64)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), c = w / W;
+    const int sub = (int)(w % W);
+    const TI *A[ND], *B[ND];
 #pragma unroll
     for (int d = 0; d < ND; ++d) { A[d] = pr.a[d]; B[d] = pr.b[d]; }
-    double acc[ND][NV];
+    double v[C];
+    if (c < nch) dot_chunk<TI, NV, ND, SH>(A, B, c * 256, (int)min((i64)256, n - c * 256), W, sub, v);
+    if (!dot_join<NV>(W, sub, sm, v) || c >= nch) return;
+    dot_fold_lanes<NV>(v);
+    if (lane < DotShape<NV>::TPR)
 #pragma unroll
-    for (int d = 0; d < ND; ++d)
+        for (int d = 0; d < ND; ++d)
 #pragma unroll
-        for (int k = 0; k < NV; ++k) acc[d][k] = 0.0;
-    constexpr int V = Shape<TI, NV>::V;
-#pragma unroll 1
-    for (int m = 0; m < 8; ++m) {
-        i64 i = c * 256 + 32 * m + lane;
-        if (i < n) {
-#pragma unroll
-            for (int d = 0; d < ND; ++d) {
-#pragma unroll
-                for (int k0 = 0; k0 < NV; k0 += V) {
-                    TI xa[V], xb[V];
-                    ld<TI, V>(A[d] + i * NV + k0, xa);
-                    ld<TI, V>(B[d] + i * NV + k0, xb);
-#pragma unroll
-                    for (int e = 0; e < V; ++e)
-                        acc[d][k0 + e] = fma((double)xa[e], (double)xb[e], acc[d][k0 + e]);
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int d = 0; d < ND; ++d)
-#pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            double v = acc[d][k];
-#pragma unroll
-            for (int off = 16; off >= 1; off >>= 1) v = dadd(v, __shfl_xor_sync(0xffffffffu, v, off));
-            if (lane == 0) part[((i64)d * NV + k) * nch + c] = v;
-        }
+            for (int e = 0; e < V; ++e) part[((i64)d * NV + lane * V + e) * nch + c] = v[d * V + e];
 }
 
-// Stage 2: block (d,k): slot t sums chunks t, t+256, ... in order from 0, then
-// the 256 slots fold pairwise (off = 128..1).
+// Stage 2 of one column and pair, by 256 threads (t = 0 .. 255, q their slots):
+// slot t sums chunks t, t+256, ... in order from 0, eight of them under way, then
+// the 256 slots fold pairwise (off = 128..1); the value is thread 0's.
+__device__ __forceinline__ double dot_slots(i64 nch, const double *__restrict__ p, int t, double *q) {
+    double a = 0.0;
+    i64 c = t;
+    for (; c + 7 * 256 < nch; c += 8 * 256) {
+        double v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = __ldcg(p + c + u * 256);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) a = dadd(a, v[u]);
+    }
+    for (; c < nch; c += 256) a = dadd(a, __ldcg(p + c));
+    q[t] = a;
+    __syncthreads();
+    double v = 0.0;
+    if (t < 32) {
+        // the folds by 128, 64 and 32 are of this lane's own slots
+        double s[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) s[u] = q[t + 32 * u];
+#pragma unroll
+        for (int off = 4; off >= 1; off >>= 1)
+#pragma unroll
+            for (int u = 0; u < off; ++u) s[u] = dadd(s[u], s[u + off]);
+        v = s[0];
+#pragma unroll
+        for (int off = 16; off >= 1; off >>= 1) v = dadd(v, __shfl_xor_sync(0xffffffffu, v, off));
+    }
+    return v;
+}
 __global__ void __launch_bounds__(256) k_dot2(i64 nch, const double *__restrict__ part,
                                               double *__restrict__ out) {
     __shared__ double q[256];
-    const double *p = part + (i64)blockIdx.x * nch;
-    double a = 0.0;
-    for (i64 c = threadIdx.x; c < nch; c += 256) a = dadd(a, p[c]);
-    q[threadIdx.x] = a;
-    __syncthreads();
-    for (int off = 128; off >= 32; off >>= 1) {
-        if (threadIdx.x < off) q[threadIdx.x] = dadd(q[threadIdx.x], q[threadIdx.x + off]);
-        __syncthreads();
-    }
-    if (threadIdx.x < 32) {
-        double v = q[threadIdx.x];
-        for (int off = 16; off >= 1; off >>= 1) v = dadd(v, __shfl_xor_sync(0xffffffffu, v, off));
-        if (threadIdx.x == 0) out[blockIdx.x] = v;
-    }
+    const double v = dot_slots(nch, part + (i64)blockIdx.x * nch, threadIdx.x, q);
+    if (threadIdx.x == 0) out[blockIdx.x] = v;
 }
 
 // Inner products in the reference's single-core order (blas.inl:561-576):
@@ -1325,7 +1319,6 @@ static void dots_t(i64 n, int nd, const void *const *a, const void *const *b, do
         if (reduce) cudaMemsetAsync(out, 0, sizeof(double) * nd * NV, s);
         return;
     }
-    unsigned g = (unsigned)((nch + 7) / 8);
     DotPairs<TI> pr;
     for (int d = 0; d < 4; ++d) {
         pr.a[d] = (const TI *)a[d < nd ? d : 0];
@@ -1342,19 +1335,15 @@ static void dots_t(i64 n, int nd, const void *const *a, const void *const *b, do
         return;
     }
     note_launch(2);
-    if (nd == 1) k_dot1<TI, NV, 1><<<g, 256, 0, s>>>(n, nch, pr, part);
-    else if (nd == 2) k_dot1<TI, NV, 2><<<g, 256, 0, s>>>(n, nch, pr, part);
-    else if (nd == 3) k_dot1<TI, NV, 3><<<g, 256, 0, s>>>(n, nch, pr, part);
-    else if constexpr (NV <= 8) k_dot1<TI, NV, 4><<<g, 256, 0, s>>>(n, nch, pr, part);
-    else {
-        // four pairs at wide NV: two passes of two pairs (register budget);
-        // each pair's partials are the same as in one pass
-        DotPairs<TI> hi;
-        for (int d = 0; d < 2; ++d) { hi.a[d] = pr.a[d + 2]; hi.b[d] = pr.b[d + 2]; hi.a[d + 2] = hi.a[d]; hi.b[d + 2] = hi.b[d]; }
-        note_launch();
-        k_dot1<TI, NV, 2><<<g, 256, 0, s>>>(n, nch, pr, part);
-        k_dot1<TI, NV, 2><<<g, 256, 0, s>>>(n, nch, hi, part + (i64)2 * NV * nch);
-    }
+    const DotSplit sp = dot_split<NV>(nch, sm_count());
+    const bool sh = nd == 3 && pr.a[1] == pr.a[0] && pr.b[1] == pr.a[0] && pr.a[2] == pr.b[0] && pr.b[2] == pr.b[0];
+#define L(ND, SH) k_dot1<TI, NV, ND, SH><<<sp.blocks, 32 * sp.warps, 0, s>>>(n, nch, sp.W, pr, part)
+    if (nd == 1) L(1, false);
+    else if (nd == 2) L(2, false);
+    else if (sh) L(3, true);
+    else if (nd == 3) L(3, false);
+    else L(4, false);
+#undef L
     if (!reduce) {
         note_launch(-1);
         return;
@@ -1577,117 +1566,139 @@ void negate(int nv, const double *in, double *out, cudaStream_t s) {
 // (same expressions, same chunk/lane/slot tree), so the fused iteration gives
 // the same bits.
 
+// E elements (16 bytes, or one where the arrays are not aligned or do not
+// divide) of a thread.
+// Bound: HBM.  One element a thread took half as long again (FP32, NV 16, 262144
+// rows: s 15.3 us, now 8.1; p 17.6, now 11.7).
 // s = 1*r + (-alpha)*v; sz (the preconditioned copy about to be formed) = 0
-template <class T, int NV>
+template <class T, int NV, int E>
 __global__ void __launch_bounds__(256) k_bicg_s(i64 total, const double *__restrict__ alpha,
                                                 const T *__restrict__ r, const T *__restrict__ v,
                                                 T *__restrict__ s, T *__restrict__ sz) {
-    i64 q = (i64)blockIdx.x * 256 + threadIdx.x;
+    const i64 q = ((i64)blockIdx.x * 256 + threadIdx.x) * E;
     if (q >= total) return;
-    int k = (int)(q % NV);
-    double na = dmul(-1.0, alpha[k]);
-    s[q] = (T)dadd(dmul(1.0, (double)r[q]), dmul(na, (double)v[q]));
-    if (sz) sz[q] = T(0);
+    T a[E], b[E], z[E];
+    ld<T, E>(r + q, a);
+    ld<T, E>(v + q, b);
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const double na = dmul(-1.0, __ldg(alpha + (int)((q + e) % NV)));
+        a[e] = (T)dadd(dmul(1.0, (double)a[e]), dmul(na, (double)b[e]));
+        z[e] = T(0);
+    }
+    st<T, E>(s + q, a);
+    if (sz) st<T, E>(sz + q, z);
 }
 
 // p = 1*r + c1*v + beta*p; pz = 0
-template <class T, int NV>
+template <class T, int NV, int E>
 __global__ void __launch_bounds__(256) k_bicg_p(i64 total, const double *__restrict__ c1,
                                                 const double *__restrict__ beta, const T *__restrict__ r,
                                                 const T *__restrict__ v, T *__restrict__ p, T *__restrict__ pz) {
-    i64 q = (i64)blockIdx.x * 256 + threadIdx.x;
+    const i64 q = ((i64)blockIdx.x * 256 + threadIdx.x) * E;
     if (q >= total) return;
-    int k = (int)(q % NV);
-    p[q] = (T)dadd(dadd(dmul(1.0, (double)r[q]), dmul(c1[k], (double)v[q])), dmul(beta[k], (double)p[q]));
-    if (pz) pz[q] = T(0);
+    T a[E], b[E], c[E], z[E];
+    ld<T, E>(r + q, a);
+    ld<T, E>(v + q, b);
+    ld_cg<T, E>(p + q, c);
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+        const int k = (int)((q + e) % NV);
+        c[e] = (T)dadd(dadd(dmul(1.0, (double)a[e]), dmul(__ldg(c1 + k), (double)b[e])),
+                       dmul(__ldg(beta + k), (double)c[e]));
+        z[e] = T(0);
+    }
+    st<T, E>(p + q, c);
+    if (pz) st<T, E>(pz + q, z);
 }
 
 // x = ac*pp + oc*ss + 1*x;  r = 1*s + (-omega)*t;  chunk partials of (r, r0)
-// in the layout of k_dot1 (warp = chunk of 256 rows, lane l sums rows
-// l + 32m, m = 0..7, then the lanes fold 16..1).
+// in the layout and order of k_dot1 (dots.cuh).
 template <class T, int NV>
-__global__ void __launch_bounds__(256) k_bicg_xr(i64 n, i64 nch, const double *__restrict__ ac,
+__global__ void __launch_bounds__(256, 2) k_bicg_xr(i64 n, i64 nch, int W, const double *__restrict__ ac,
                                                  const double *__restrict__ oc, const double *__restrict__ omega,
                                                  const T *__restrict__ pp, const T *__restrict__ ss,
                                                  T *__restrict__ x, const T *__restrict__ s,
                                                  const T *__restrict__ t, T *__restrict__ r,
                                                  const T *__restrict__ r0, double *__restrict__ part) {
-    const int lane = threadIdx.x & 31;
-    const i64 c = (i64)blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (c >= nch) return;
-    constexpr int V = Shape<T, NV>::V;
-    double acc[NV];
+    typedef DotShape<NV> S;
+    constexpr int V = S::V, U = sizeof(T) * V <= 8 ? 4 : 2;
+    __shared__ double sm[8 * V * 32];
+    const int lane = threadIdx.x & 31, q = lane / S::TPR, k0 = lane % S::TPR * V, JW = S::TPR / W;
+    const i64 w = (i64)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), c = w / W;
+    const int sub = (int)(w % W);
+    double fa[V], fo[V], fw[V], acc[V];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) acc[k] = 0.0;
+    for (int e = 0; e < V; ++e) {
+        fa[e] = __ldg(ac + k0 + e);
+        fo[e] = __ldg(oc + k0 + e);
+        fw[e] = dmul(-1.0, __ldg(omega + k0 + e));
+        acc[e] = 0.0;
+    }
+    DotStack<S::LOG, V> tree;
+    if (c < nch)
 #pragma unroll 1
-    for (int m = 0; m < 8; ++m) {
-        i64 i = c * 256 + 32 * m + lane;
-        if (i >= n) continue;
+        for (int i = 0; i < JW; ++i) {
+            const i64 row = c * 256 + dot_bitrev<S::LOG>(sub * JW + i) * S::RPI + q;
 #pragma unroll
-        for (int k0 = 0; k0 < NV; k0 += V) {
-            const i64 o = i * NV + k0;
-            T a[V], b[V], xx[V], sv[V], tv[V], z[V], xo[V], ro[V];
-            ld<T, V>(pp + o, a);
-            ld<T, V>(ss + o, b);
-            ld_cg<T, V>(x + o, xx);
-            ld<T, V>(s + o, sv);
-            ld<T, V>(t + o, tv);
-            ld<T, V>(r0 + o, z);
+            for (int e = 0; e < V; ++e) acc[e] = 0.0;
 #pragma unroll
-            for (int e = 0; e < V; ++e) {
-                const int k = k0 + e;
-                xo[e] = (T)dadd(dadd(dmul(__ldg(ac + k), (double)a[e]), dmul(__ldg(oc + k), (double)b[e])),
-                                dmul(1.0, (double)xx[e]));
-                const double nw = dmul(-1.0, __ldg(omega + k));
-                ro[e] = (T)dadd(dmul(1.0, (double)sv[e]), dmul(nw, (double)tv[e]));
-                acc[k] = fma((double)ro[e], (double)z[e], acc[k]);
+            for (int m = 0; m < 8; m += U) {
+                T a[U][V], b[U][V], xx[U][V], sv[U][V], tv[U][V], z[U][V];
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    // past the end: the last row again, neither stored nor added
+                    const i64 o = min(row + (m + u) * 32, n - 1) * NV + k0;
+                    ld<T, V>(pp + o, a[u]);
+                    ld<T, V>(ss + o, b[u]);
+                    ld_cg<T, V>(x + o, xx[u]);
+                    ld<T, V>(s + o, sv[u]);
+                    ld<T, V>(t + o, tv[u]);
+                    ld<T, V>(r0 + o, z[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    if (row + (m + u) * 32 >= n) break;
+                    const i64 o = (row + (m + u) * 32) * NV + k0;
+                    T xo[V], ro[V];
+#pragma unroll
+                    for (int e = 0; e < V; ++e) {
+                        xo[e] = (T)dadd(dadd(dmul(fa[e], (double)a[u][e]), dmul(fo[e], (double)b[u][e])),
+                                        dmul(1.0, (double)xx[u][e]));
+                        ro[e] = (T)dadd(dmul(1.0, (double)sv[u][e]), dmul(fw[e], (double)tv[u][e]));
+                        acc[e] = fma((double)ro[e], (double)z[u][e], acc[e]);
+                    }
+                    st<T, V>(x + o, xo);
+                    st<T, V>(r + o, ro);
+                }
             }
-            st<T, V>(x + o, xo);
-            st<T, V>(r + o, ro);
+            tree.push(i, acc);
         }
-    }
+    if (!dot_join<NV>(W, sub, sm, acc) || c >= nch) return;
+    dot_fold_lanes<NV>(acc);
+    if (lane < S::TPR)
 #pragma unroll
-    for (int k = 0; k < NV; ++k) {
-        double v = acc[k];
-#pragma unroll
-        for (int off = 16; off >= 1; off >>= 1) v = dadd(v, __shfl_xor_sync(0xffffffffu, v, off));
-        if (lane == 0) part[(i64)k * nch + c] = v;
-    }
+        for (int e = 0; e < V; ++e) part[(i64)(k0 + e) * nch + c] = acc[e];
 }
 
-// Stage 2 of the inner products (the k_dot2 tree) for all nd pairs of one
-// column k per block, then that column's scalar recurrence.
+// Stage 2 of the inner products (the k_dot2 tree) for all nd <= 3 pairs of one
+// column k per block, 256 threads each, then that column's scalar recurrence.
 enum { EPI_ALPHA = 0, EPI_OMEGA = 1, EPI_BETA = 2 };
 template <int EPI>
 __device__ __forceinline__ void bicg_epi_col(int k, const double *val, const BicgScalars &sc);
 template <int EPI>
-__global__ void __launch_bounds__(256) k_dot2_epi(i64 nch, int nd, int nv, const double *__restrict__ part,
+__global__ void __launch_bounds__(768) k_dot2_epi(i64 nch, int nd, int nv, const double *__restrict__ part,
                                                   double *__restrict__ out, BicgScalars sc) {
-    __shared__ double q[256];
+    __shared__ double q[3 * 256];
     __shared__ double val[4];
-    const int k = blockIdx.x;
-    for (int d = 0; d < nd; ++d) {
-        const double *p = part + ((i64)d * nv + k) * nch;
-        double a = 0.0;
-        for (i64 c = threadIdx.x; c < nch; c += 256) a = dadd(a, p[c]);
-        q[threadIdx.x] = a;
-        __syncthreads();
-        for (int off = 128; off >= 32; off >>= 1) {
-            if (threadIdx.x < off) q[threadIdx.x] = dadd(q[threadIdx.x], q[threadIdx.x + off]);
-            __syncthreads();
-        }
-        if (threadIdx.x < 32) {
-            double v = q[threadIdx.x];
-            for (int off = 16; off >= 1; off >>= 1) v = dadd(v, __shfl_xor_sync(0xffffffffu, v, off));
-            if (threadIdx.x == 0) {
-                val[d] = v;
-                out[(i64)d * nv + k] = v;
-            }
-        }
-        __syncthreads();
+    const int k = blockIdx.x, d = threadIdx.x >> 8, t = threadIdx.x & 255;
+    const double v = dot_slots(nch, part + ((i64)d * nv + k) * nch, t, q + d * 256);
+    if (t == 0) {
+        val[d] = v;
+        out[(i64)d * nv + k] = v;
     }
-    if (threadIdx.x != 0) return;
-    bicg_epi_col<EPI>(k, val, sc);
+    __syncthreads();
+    if (threadIdx.x == 0) bicg_epi_col<EPI>(k, val, sc);
 }
 
 // the recurrence alone, from reduced values vals[d*nv + k] (one thread per column)
@@ -2210,16 +2221,23 @@ static void bicg_groups_t(int grp, i64 n, const BicgScalars &sc, const void *a0,
                           const void *a3, const void *a4, void *a5, const void *a6, double *part, cudaStream_t s) {
     const i64 tot = n * NV;
     if (tot <= 0) return;
-    const unsigned g = (unsigned)((tot + 255) / 256);
+    constexpr int E = 16 / (int)sizeof(T);
+    const bool wide = tot % E == 0 && (((uintptr_t)a0 | (uintptr_t)a1 | (uintptr_t)a2 | (uintptr_t)a5) & 15) == 0;
+    const unsigned g = (unsigned)((wide ? tot / E + 255 : tot + 255) / 256);
     note_launch();
     if (grp == 0) {
-        k_bicg_s<T, NV><<<g, 256, 0, s>>>(tot, sc.alpha, (const T *)a0, (const T *)a1, (T *)a2, (T *)a5);
+        if (wide) k_bicg_s<T, NV, E><<<g, 256, 0, s>>>(tot, sc.alpha, (const T *)a0, (const T *)a1, (T *)a2, (T *)a5);
+        else k_bicg_s<T, NV, 1><<<g, 256, 0, s>>>(tot, sc.alpha, (const T *)a0, (const T *)a1, (T *)a2, (T *)a5);
     } else if (grp == 1) {
-        k_bicg_p<T, NV><<<g, 256, 0, s>>>(tot, sc.c1, sc.beta, (const T *)a0, (const T *)a1, (T *)a2, (T *)a5);
+        if (wide)
+            k_bicg_p<T, NV, E><<<g, 256, 0, s>>>(tot, sc.c1, sc.beta, (const T *)a0, (const T *)a1, (T *)a2, (T *)a5);
+        else
+            k_bicg_p<T, NV, 1><<<g, 256, 0, s>>>(tot, sc.c1, sc.beta, (const T *)a0, (const T *)a1, (T *)a2, (T *)a5);
     } else {
         const i64 nch = (n + 255) / 256;
-        k_bicg_xr<T, NV><<<(unsigned)((nch + 7) / 8), 256, 0, s>>>(
-            n, nch, sc.ac, sc.oc, sc.omega, (const T *)a0, (const T *)a1, (T *)a2, (const T *)a3, (const T *)a4,
+        const DotSplit sp = dot_split<NV>(nch, sm_count());
+        k_bicg_xr<T, NV><<<sp.blocks, 32 * sp.warps, 0, s>>>(
+            n, nch, sp.W, sc.ac, sc.oc, sc.omega, (const T *)a0, (const T *)a1, (T *)a2, (const T *)a3, (const T *)a4,
             (T *)a5, (const T *)a6, part);
     }
 }
@@ -2267,9 +2285,9 @@ void dot_reduce_epi(int epi, i64 n, int nd, int nv, const double *part, double *
                     cudaStream_t s) {
     const i64 nch = (n + 255) / 256;
     note_launch();
-    if (epi == EPI_ALPHA) k_dot2_epi<EPI_ALPHA><<<nv, 256, 0, s>>>(nch, nd, nv, part, out, sc);
-    else if (epi == EPI_OMEGA) k_dot2_epi<EPI_OMEGA><<<nv, 256, 0, s>>>(nch, nd, nv, part, out, sc);
-    else k_dot2_epi<EPI_BETA><<<nv, 256, 0, s>>>(nch, nd, nv, part, out, sc);
+    if (epi == EPI_ALPHA) k_dot2_epi<EPI_ALPHA><<<nv, 256 * nd, 0, s>>>(nch, nd, nv, part, out, sc);
+    else if (epi == EPI_OMEGA) k_dot2_epi<EPI_OMEGA><<<nv, 256 * nd, 0, s>>>(nch, nd, nv, part, out, sc);
+    else k_dot2_epi<EPI_BETA><<<nv, 256 * nd, 0, s>>>(nch, nd, nv, part, out, sc);
 }
 
 void bicg_epi(int epi, int nv, const double *vals, const BicgScalars &sc, cudaStream_t s) {
