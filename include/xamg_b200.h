@@ -201,9 +201,10 @@ int xamg_csr_spmv(int prec, int nv, int64_t n, const int *rp, const int *ci, con
  * a time; 5, 6 = staged entries with a plain row loop unrolled 4 or 8 times;
  * 8 = a warp's rows side by side with their entries staged a step ahead;
  * 10 + k = staged streaming kernel walking k tiles per CTA; -1 = default (by
- * row width, and for the library's own operators by rows and entries).  Under -1 and 7 the products
- * of operators that have a shifted-row run plan (below) use the run kernel
- * (7 elsewhere = the default).  The setting belongs to the calling host
+ * row width, and for the library's own operators by rows and entries).
+ * Under 7, and under -1 where it is the faster one, the products of operators
+ * that have a shifted-row run plan (below) use the run kernel (7 elsewhere =
+ * the default).  The setting belongs to the calling host
  * thread; a batch's autotuned choices are held by its own operators and are
  * not affected by it.  Returns the previous setting. */
 int xamg_spmv_set_variant(int variant);

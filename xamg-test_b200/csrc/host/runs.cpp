@@ -159,13 +159,24 @@ void RunPlan::add_values(const HostCsr &h, Prec p) {
     }
 }
 
+// Whether an operator's run plan is its default product.  From 128 bytes a row
+// it is; with 64 the CSR kernels are ahead on small operators and on short rows
+// (us, runs / best CSR kernel: FP32 NV 16 27-point 32^3 7.5 / 6.5, 64^3 24 / 33,
+// 7-point 64^3 14.1 / 11.4, 100^3 55.7 / 58.8; FP64 NV 8 27-point 64^3 38.9 / 36.4,
+// with b - A x 49.8 / 38.1, 100^3 133 / 134 and 152 / 144, 128^3 239 / 272 and
+// 282 / 292, 7-point 100^3 76 / 71).
+static bool runs_by_default(Prec p, int nv, i64 n, i64 nnz) {
+    if (nv * (i64)prec_size(p) >= 128) return true;
+    return nnz >= 16 * n && n > (p == Prec::F64 ? 1000000 : 65536);
+}
+
 void DCsr::spmv(Prec p, int nv, const void *x, void *y, int mode, const void *b, cudaStream_t s) const {
     const int own = variant[p == Prec::F64 ? 0 : 1];
     const int var = own >= 0 ? own : xk::get_spmv_variant();
     const double sv = (double)prec_size(p);
     // x read once, y written, y or b read for modes 1 and 2
     const double xy = (double)ncols * nv * sv + (double)n * nv * sv * (mode >= 1 ? 2 : 1);
-    if ((var < 0 || var == 7) && runs.has(p) && xk::spmv_runs_supported(p, nv)) {
+    if (((var < 0 && runs_by_default(p, nv, n, nnz)) || var == 7) && runs.has(p) && xk::spmv_runs_supported(p, nv)) {
         // run format: values once, 4 B per segment, 20 B per chunk (descriptor
         // and its share of the tile offsets)
         KTimeScope kt(KClass::SPMV, n, (double)nnz * sv + 4.0 * runs.nseg + 20.0 * runs.nchunks + xy, s);

@@ -576,6 +576,15 @@ __device__ __forceinline__ void run_rows(const int4 cd, int smax, const int *sg,
         for (int q = 0; q < R; ++q)
             if (q < cd.y) ld<T, V>(y + ((i64)cd.x + q) * NV + l * V, acc[q]);
     }
+    if (MODE == 2 && NV * sizeof(T) >= 128) {
+        // b is wanted after the last segment, when there is nothing left to hide its
+        // latency behind: its lines are asked for now (27-point 64^3, us before and
+        // after: FP64 NV 16 69.4 and 64.9, NV 32 108.1 and 97.9, FP32 NV 32 61.7 and
+        // 56.9; rows of 64 bytes gain nothing, FP32 NV 16 29.9 and 30.7)
+        const char *line = reinterpret_cast<const char *>(b + (i64)cd.x * NV);
+        for (int o = l * 128; o < cd.y * NV * (int)sizeof(T); o += Shape<T, NV>::TPR * 128)
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(line + o));
+    }
     auto seg = [&](int s) { return s < cd.w ? (SMEM ? sg[4 * s] : __ldcs(sg + 4 * s)) : 0; };
     int e = 0;
     int sc = seg(0);

@@ -35,7 +35,8 @@ void spmv(Prec p, int nv, i64 n, const int *rp, const int *ci, const void *val, 
 // 8 times; 8 = rows side by side, entries staged a step ahead; 10 + k =
 // streaming kernel walking k tiles per CTA; -1 = default (by width, rows and,
 // where given, entries).  All give identical results.
-// Operators with a shifted-row run plan use the run kernel under -1 and 7
+// Operators with a shifted-row run plan use the run kernel under 7, and under
+// -1 where it is the faster one
 // (7 elsewhere = the default).  The setting is per host thread; an operator
 // can also carry its own choice (DCsr::variant), which takes precedence.
 void set_spmv_variant(int v);
