@@ -36,8 +36,8 @@ def laplace(n):
     return np.array(rp, np.int32), np.array(ci, np.int32), np.array(v)
 
 
-def run(arrays, B, iters, timed):
-    spec = util.amg_params(precond_mg=False, max_iters=iters)
+def run(arrays, B, iters, timed, meta=None):
+    spec = util.amg_params(precond_mg=False, max_iters=iters, meta=meta)
     n, nv = B.shape
     xamg.set_nv(nv)
     A = xamg.Matrix(xamg.CsrMatrix.from_arrays(*arrays))
@@ -84,5 +84,20 @@ def test_iterations_continue_over_launches(gpu):
     x, it, hist = run(arrays, B, 600, False)
     x1, it1, hist1 = run(arrays, B, 600, True)
     assert it == it1 == 600
+    np.testing.assert_array_equal(hist, hist1)
+    np.testing.assert_array_equal(x, x1)
+
+
+@pytest.mark.parametrize("nv", [1, 2, 4, 8, 16, 32])
+def test_iterations_in_fp32(gpu, nv):
+    # the inner solver of a refinement with reduced precision
+    meta = {"method": "IterativeRefinement", "max_iters": 20, "abs_tolerance": 0.0, "rel_tolerance": 1e-9,
+            "subsolver_reduced_precision": True, "inner_rel_tolerance": 1e-4,
+            "convergence_details": "check-L2,noprint"}
+    arrays = band(1500, 3, nv, 7)
+    B = np.random.default_rng(nv).uniform(-1, 1, (1500, nv))
+    x, it, hist = run(arrays, B, 60, False, meta)
+    x1, it1, hist1 = run(arrays, B, 60, True, meta)
+    assert it == it1 > 0
     np.testing.assert_array_equal(hist, hist1)
     np.testing.assert_array_equal(x, x1)

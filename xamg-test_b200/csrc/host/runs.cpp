@@ -164,8 +164,12 @@ void RunPlan::add_values(const HostCsr &h, Prec p) {
 // (us, runs / best CSR kernel: FP32 NV 16 27-point 32^3 7.5 / 6.5, 64^3 24 / 33,
 // 7-point 64^3 14.1 / 11.4, 100^3 55.7 / 58.8; FP64 NV 8 27-point 64^3 38.9 / 36.4,
 // with b - A x 49.8 / 38.1, 100^3 133 / 134 and 152 / 144, 128^3 239 / 272 and
-// 282 / 292, 7-point 100^3 76 / 71).
+// 282 / 292, 7-point 100^3 76 / 71).  Coarse operators, of 43 to 160 entries a
+// row, have few rows in common runs: there the rows side by side are ahead at
+// every width (the products of a hierarchy's level, FP32 NV 32 63049 rows 77 / 37,
+// 250000 rows 92 / 69, NV 16 250000 rows 55 / 46).
 static bool runs_by_default(Prec p, int nv, i64 n, i64 nnz) {
+    if (nnz >= 32 * n) return false;
     if (nv * (i64)prec_size(p) >= 128) return true;
     return nnz >= 16 * n && n > (p == Prec::F64 ? 1000000 : 65536);
 }

@@ -443,7 +443,9 @@ int sm_count() {
 //   shorter rows: GB 4 (7-point 113x97x101 FP32 NV 8 60 / 33 / 43 / 45, FP64 NV 16
 //   157 / 150 / 166 / 154), in FP64 with one thread a row GB 8 (NV 1 32 / 23 / 21 / 26);
 //   not known: as for short rows, wide ones tile-staged (27-point 100^3 FP64 NV 16
-//   331 against 222, 7-point 150 against 154).
+//   331 against 222, 7-point 150 against 154) or, few of them, side by side
+//   (FP64 NV 16: 576 rows of 6 2.4 against 3.1, 1320 of 22 3.2 against 4.4, 300 of
+//   38 6.2 against 12.8; at 19683 rows of 7 4.7 against 4.0).
 template <class T, int NV>
 static int default_variant(i64 n, i64 nnz) {
     constexpr int TPR = Shape<T, NV>::TPR;
@@ -453,7 +455,7 @@ static int default_variant(i64 n, i64 nnz) {
         return TPR <= 2 || nnz >= 32 * n || n <= 20000 ? 8 : 6;
     }
     if (TPR == 1) return f64 ? 1 : 0;
-    return TPR >= 4 && nnz < 0 ? 6 : 0;
+    return TPR >= 4 && nnz < 0 ? (n <= 8192 ? 8 : 6) : 0;
 }
 
 template <class T, int NV>
