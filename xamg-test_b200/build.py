@@ -39,7 +39,7 @@ def _newer(src, dst):
 
 def build_library(verbose=False):
     os.makedirs(BUILD, exist_ok=True)
-    headers = [os.path.join(CSRC, f) for f in ("kernels.cuh", "dots.cuh")] + [
+    headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".cuh", ".h"))] + [
         os.path.join(CSRC, "host", f) for f in os.listdir(os.path.join(CSRC, "host")) if f.endswith(".h")
     ] + [os.path.join(ROOT, "include", f) for f in os.listdir(os.path.join(ROOT, "include"))]
     hdr_time = max(os.path.getmtime(h) for h in headers)

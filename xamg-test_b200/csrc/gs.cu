@@ -33,6 +33,7 @@
 //
 // Every wait is bounded by a wall-clock limit; on expiry the error word is set
 // and the CTA leaves after its own copies in flight have landed.
+#include "gs_columns.h"
 #include "kernels.cuh"
 #include <algorithm>
 #include <climits>
@@ -335,6 +336,9 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_gs_block(const __grid_constant
     const int q = lane / TPR, l = lane % TPR;
     const int b = blockIdx.x;
     const int xb = b * brows;  // first row of the block
+    // what a column may be at most: with the x tile one past a full block (its row
+    // of zeros), else one past the rows that this block has
+    const int lim = XS ? brows : gs_block_rows(n, brows, b);
     const int stage_bytes = eb * (4 + (int)sizeof(T));
     unsigned char *sbuf = dyn + (size_t)warp * 2 * stage_bytes;
     const unsigned sba = smem_u32(sbuf);
@@ -358,7 +362,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_gs_block(const __grid_constant
 #pragma unroll
     for (int e = 0; e < V; ++e) rl[e] = relax[l * V + e];
     __syncthreads();
-    // x of column c of the block (brows: a row of zeros), this lane's columns: a
+    // x of column c of the block (lim: a row of zeros), this lane's columns: a
     // column becomes a shared-memory address (XS), or stays a column
     constexpr int RB = NV * (int)sizeof(T);
     const unsigned xsa = smem_u32(xs) + l * V * (int)sizeof(T);
@@ -367,7 +371,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_gs_block(const __grid_constant
     auto where = [&](int c) -> int { return XS ? (int)(xsa + (unsigned)c * RB) : c; };
     auto xld = [&](int w, T(&r)[V]) {
         if constexpr (XS) xls((unsigned)w, r);
-        else xlg(w < brows ? xga + (size_t)w * RB : zga, r);
+        else xlg(w < lim ? xga + (size_t)w * RB : zga, r);
     };
     for (int pass = 0; pass < 2; ++pass) {
         const GsDir &d = pass ? bw : fw;
@@ -406,7 +410,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_gs_block(const __grid_constant
             auto ldc = [&](int g, int (&c)[4]) {
                 lds4(ca + r16 * g, r16, c);
 #pragma unroll
-                for (int u = 0; u < 4; ++u) c[u] = where((int)min((unsigned)c[u], (unsigned)brows));
+                for (int u = 0; u < 4; ++u) c[u] = where(gs_block_column(c[u], lim));
             };
             auto ldv = [&](int g, T(&v)[4]) { lds4(va + (unsigned)(sizeof(T) / 4) * r16 * g, r16, v); };
             auto ldx = [&](const int (&c)[4], T(&xv)[4][V]) {
@@ -447,9 +451,9 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_gs_block(const __grid_constant
                     g1 = cnt >> 2;
                 }
                 // before the wait: the first two groups' addresses.  Loads run up
-                // to three groups past the segment's end (their columns are
-                // clamped to the block and nothing uses them), so that the loop
-                // has one branch a group.
+                // to three groups past the segment's end (their columns are whatever
+                // the stage holds there, clamped to the block's own rows, and nothing
+                // uses them), so that the loop has one branch a group.
                 ldc(g, c0);
                 ldc(g + 1, c1);
                 if (last || longrow)
