@@ -261,9 +261,10 @@ int xamg_gs_plan_levels(void *plan, int *nlev /* [2] */, int *lf, int *lb);
 /* Self-test of the device-side bounded waits (an extension): makes a wait
  * run out on purpose with a limit of limit_s seconds (at most 2) and reports
  * it the way a solve does, code 3 with the message in XAMG_b200_last_error.
- * which = 0: cooperative grid of ncta (2..64) CTAs whose barrier misses one
- * arrival; 1: an mbarrier phase that nothing completes.  The device stays
- * usable afterwards. */
+ * which = 0: an element of a vector that ncta - 1 CTAs (ncta 2..64) read until
+ * it is written, which it is not; 1: an mbarrier phase that nothing completes;
+ * 2: a Gauss-Seidel block sweep of ncta blocks, one of which waits for an item
+ * that does not exist.  The device stays usable afterwards. */
 int XAMG_b200_wait_selftest(int which, int ncta, double limit_s);
 /* Slots of the shared-memory x window of each sweep direction of a hybrid
  * plan with values, as the warp-per-block kernel would use it (0: no window). */

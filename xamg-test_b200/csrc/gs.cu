@@ -43,7 +43,7 @@ namespace xk {
 
 namespace {
 
-constexpr unsigned long long kLimitNs = 1000000000ull;  // 1 s
+constexpr unsigned long long kLimitNs = kGsWaitNs;
 
 __device__ __forceinline__ unsigned long long now_ns() {
     unsigned long long t;
@@ -227,7 +227,7 @@ __device__ __forceinline__ bool mbar_try(unsigned long long *bar, unsigned parit
 // bounded wait on an mbarrier phase; false on expiry (then, or when another
 // warp's wait has expired, *fail is set)
 __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, unsigned parity, volatile int *fail,
-                                          unsigned long long limit = kLimitNs) {
+                                          unsigned long long limit) {
     if (mbar_try(bar, parity)) return true;
     const unsigned long long t0 = now_ns();
     unsigned spins = 0;
@@ -326,7 +326,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_gs_block(const __grid_constant
                                                                    const __grid_constant__ GsDir bw,
                                                                    const T *__restrict__ t, T *x,
                                                                    const T *__restrict__ relax, int brows, int n,
-                                                                   int eb, int split, int *err) {
+                                                                   int eb, int split, unsigned long long limit,
+                                                                   int *err) {
     constexpr int V = Sh<T, NV>::V, TPR = Sh<T, NV>::TPR, RPW = 32 / TPR, W = NT / 32;
     static_assert(W + 2 <= kRing, "ring parities");
     extern __shared__ __align__(128) unsigned char dyn[];
@@ -434,7 +435,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_gs_block(const __grid_constant
             const bool longrow = ne > eb;
             const int k0 = longrow ? 0 : a.k0();
             int done = 0;  // long row: entries summed
-            if (lev > 1 && !longrow) ok = mbar_wait(bar + (lev - 2) % kRing, (lev - 2) / kRing & 1, &s_fail);
+            if (lev > 1 && !longrow) ok = mbar_wait(bar + (lev - 2) % kRing, (lev - 2) / kRing & 1, &s_fail, limit);
             xld(where(r.row - xb), xo);  // only this row's own item writes it
             int g = 0, g1 = k0 > 0 ? k0 : a.groups();
             bool last = k0 == 0;
@@ -457,8 +458,10 @@ __global__ void __launch_bounds__(NT, 512 / NT) k_gs_block(const __grid_constant
                 ldc(g, c0);
                 ldc(g + 1, c1);
                 if (last || longrow)
-                    if (lev > 0) ok = ok && mbar_wait(bar + (lev - 1) % kRing, (lev - 1) / kRing & 1, &s_fail);
-                if (!__all_sync(0xffffffffu, ok)) break;
+                    if (lev > 0) ok = ok && mbar_wait(bar + (lev - 1) % kRing, (lev - 1) / kRing & 1, &s_fail, limit);
+                // one verdict for the warp: its lanes leave together or not at all
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
                 ldx(c0, x0);
                 ldx(c1, x1);
                 ldv(g, v0);
@@ -677,18 +680,19 @@ static int item_split(int rows, int rpw) {
 
 template <class T, int NV, bool XS, int NT>
 static cudaError_t gs_block_l(int nblocks, const GsDir &f, const GsDir &b, const T *t, T *x, const T *relax, int brows,
-                              int n, int eb, int split, size_t smem, int *err, cudaStream_t s) {
+                              int n, int eb, int split, size_t smem, unsigned long long limit, int *err, cudaStream_t s) {
     auto k = k_gs_block<T, NV, XS, NT>;
     // the limit belongs to the kernel: set for every launch (sizes differ)
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k<<<nblocks, NT, smem, s>>>(f, b, t, x, relax, brows, n, eb, split, err);
+    k<<<nblocks, NT, smem, s>>>(f, b, t, x, relax, brows, n, eb, split, limit, err);
     return cudaGetLastError();
 }
 
 template <class T, int NV>
 static cudaError_t gs_block_t(int nblocks, const GsDir &f, const GsDir &b, const void *t, void *x, const void *relax,
-                              i64 brows, i64 n, int emax, int *err, bool *tile, cudaStream_t s) {
+                              i64 brows, i64 n, int emax, int *err, bool *tile, cudaStream_t s,
+                              unsigned long long limit) {
     const int eb = std::min(std::max(emax, 8), kStageMax), split = item_split(f.rows, 32 / Sh<T, NV>::TPR);
     // blocks per SM that must be resident for one wave, and the threads of a
     // CTA so that their registers fit
@@ -699,7 +703,7 @@ static cudaError_t gs_block_t(int nblocks, const GsDir &f, const GsDir &b, const
     *tile = stage + tl + 1280 <= (size_t)kSmemMax / per;
     note_launch();
 #define GO(XS, NT) gs_block_l<T, NV, XS, NT>(nblocks, f, b, (const T *)t, (T *)x, (const T *)relax, (int)brows, (int)n, \
-                                             eb, split, stage + (XS ? tl : 0), err, s)
+                                             eb, split, stage + (XS ? tl : 0), limit, err, s)
     if (nt == 512) return *tile ? GO(true, 512) : GO(false, 512);
     if (nt == 256) return *tile ? GO(true, 256) : GO(false, 256);
     return *tile ? GO(true, 128) : GO(false, 128);
@@ -738,13 +742,14 @@ static cudaError_t gs_flow_t(const GsDir &d, int nitems, int nlev, int forward, 
     }
 
 cudaError_t gs_sweep_block(Prec p, int nv, int nblocks, const GsDir &f, const GsDir &b, const void *t, void *x,
-                           const void *relax, i64 brows, i64 n, int emax, int *err, bool *tile, cudaStream_t s) {
+                           const void *relax, i64 brows, i64 n, int emax, int *err, bool *tile, cudaStream_t s,
+                           unsigned long long limit_ns) {
     if (p == Prec::F64) {
-#define F(NV) gs_block_t<double, NV>(nblocks, f, b, t, x, relax, brows, n, emax, err, tile, s)
+#define F(NV) gs_block_t<double, NV>(nblocks, f, b, t, x, relax, brows, n, emax, err, tile, s, limit_ns)
         NV_SWITCH(nv, F)
 #undef F
     } else {
-#define F(NV) gs_block_t<float, NV>(nblocks, f, b, t, x, relax, brows, n, emax, err, tile, s)
+#define F(NV) gs_block_t<float, NV>(nblocks, f, b, t, x, relax, brows, n, emax, err, tile, s, limit_ns)
         NV_SWITCH(nv, F)
 #undef F
     }

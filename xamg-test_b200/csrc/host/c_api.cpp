@@ -862,19 +862,54 @@ int xamg_gs_plan_slots(void *plan, int *nslots) {
         nslots[1] = g.has_lcsr ? g.lc[1].nslots : 0;
     });
 }
+// A block sweep of ncta blocks (5-point 32 x 32 each) whose first block's
+// barriers expect one item more than there is.
+static cudaError_t stuck_block_sweep(int ncta, unsigned long long limit_ns, int *err, cudaStream_t s) {
+    const int side = 32, rows = side * side, nv = 4;
+    HostCsr A;
+    A.n = A.ncols = (i64)rows * ncta;
+    A.rp.assign(1, 0);
+    for (i64 i = 0; i < A.n; ++i) {
+        const int y = (int)(i % rows) / side, x = (int)(i % side);
+        auto entry = [&](i64 c, double v) { A.ci.push_back((int)c), A.v.push_back(v); };
+        if (y > 0) entry(i - side, -1.0);
+        if (x > 0) entry(i - 1, -1.0);
+        entry(i, 4.0);
+        if (x < side - 1) entry(i + 1, -1.0);
+        if (y < side - 1) entry(i + side, -1.0);
+        A.rp.push_back((int)A.ci.size());
+    }
+    GsPlan g;
+    g.build(A, rows, GsMode::BLOCKS);
+    g.build_lcsr(A, Prec::F64, nv);
+    int items = 0;
+    XCUDA(cudaMemcpy(&items, g.lc[0].imax.p, sizeof(int), cudaMemcpyDeviceToHost));
+    ++items;
+    XCUDA(cudaMemcpy(g.lc[0].imax.p, &items, sizeof(int), cudaMemcpyHostToDevice));
+    const size_t vec = sizeof(double) * A.n * nv;
+    DBuf b(vec), x(vec), relax(sizeof(double) * nv);
+    for (DBuf *d : {&b, &x, &relax}) XCUDA(cudaMemsetAsync(d->p, 0, d->bytes, s));
+    XCUDA(cudaMemsetAsync(err, 0, sizeof(int), s));
+    bool tile = false;
+    const cudaError_t e = xk::gs_sweep_block(Prec::F64, nv, g.nblocks, g.dir(0), g.dir(1), b.p, x.p, relax.p, g.brows, g.n,
+                                             std::max(g.lc[0].ientries, g.lc[1].ientries), err, &tile, s, limit_ns);
+    XCUDA(cudaStreamSynchronize(s));
+    return e;
+}
 int XAMG_b200_wait_selftest(int which, int ncta, double limit_s) {
     return guard([&] {
-        XCHECK(which == 0 || which == 1, "which must be 0 (unwritten element) or 1 (mbarrier)");
+        XCHECK(which >= 0 && which <= 2, "which must be 0 (unwritten element), 1 (mbarrier) or 2 (block sweep)");
         XCHECK(ncta >= 2 && ncta <= 64, "ncta must be 2..64");
         XCHECK(limit_s > 0.0 && limit_s <= 2.0, "limit must be in (0, 2] seconds");
         cudaStream_t s = ctx().stream;
         DBuf words(256), err(sizeof(int));
-        XCUDA(xk::wait_selftest(which, ncta, (unsigned long long)(limit_s * 1e9), words.as<unsigned>(),
-                                err.as<int>(), s));
+        const unsigned long long limit_ns = (unsigned long long)(limit_s * 1e9);
+        if (which == 2) XCUDA(stuck_block_sweep(ncta, limit_ns, err.as<int>(), s));
+        else XCUDA(xk::wait_selftest(which, ncta, limit_ns, words.as<unsigned>(), err.as<int>(), s));
         XCUDA(cudaStreamSynchronize(s));
         int h = 0;
         XCUDA(cudaMemcpy(&h, err.p, sizeof(int), cudaMemcpyDeviceToHost));
-        if (h) throw Error(std::string(which == 0 ? "unwritten element" : "mbarrier") +
+        if (h) throw Error(std::string(which == 0 ? "unwritten element" : which == 1 ? "mbarrier" : "block sweep") +
                                ": bounded wait expired on the device (error word " + std::to_string(h) + ")",
                            3);
     });

@@ -108,16 +108,19 @@ struct GsDir {
     const void *lva, *linvd;
     int rows;
 };
+// limit of the sweeps' waits
+constexpr unsigned long long kGsWaitNs = 1000000000ull;  // 1 s
 // most rows of a warp; entries of an item beyond which its rows are fewer (a
 // single row may have more)
 int gs_rows_per_item(Prec p, int nv);
 int gs_item_entries();
 // Forward and backward sweep of every block in one launch, one CTA per block
-// (512 threads when there is at most one block per SM, else 256).  emax: the
-// most entries of one item.  *tile: whether the x tile was in shared memory.
-// An expired wait sets *err.
+// (512 threads when there is at most one block per SM, 256 with two, else 128).
+// emax: the most entries of one item.  *tile: whether the x tile was in shared
+// memory.  A wait that takes longer than limit_ns sets *err.
 cudaError_t gs_sweep_block(Prec p, int nv, int nblocks, const GsDir &f, const GsDir &b, const void *t, void *x,
-                           const void *relax, i64 brows, i64 n, int emax, int *err, bool *tile, cudaStream_t s);
+                           const void *relax, i64 brows, i64 n, int emax, int *err, bool *tile, cudaStream_t s,
+                           unsigned long long limit_ns = kGsWaitNs);
 // One single-process sweep on the whole device: xin (values before the sweep)
 // to xout, which the call fills with a sentinel first (distinct vectors).
 cudaError_t gs_sweep_flow(Prec p, int nv, const GsDir &d, int nitems, int nlev, int forward, const void *t,
