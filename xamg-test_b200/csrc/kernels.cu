@@ -1759,7 +1759,7 @@ __device__ __forceinline__ void bicg_epi_col(int k, const double *val, const Bic
 // only where a product needs all rows: at the three inner products, whose chunk
 // partials are also the barrier.  A partial is published in two 64-bit words of
 // 32 value bits and the iteration's number each, after a fence behind the CTA's
-// vector stores (by a thread that has no partial to sum); every CTA polls all
+// vector stores by the same thread; every CTA polls all
 // partials of a column, one warp per column and pair, folds them in the tree of
 // k_dot2, and computes the scalar recurrences for itself.  FLY: the products form
 // s = r - alpha v and p = r + c1 v + beta p of the rows they gather as they go
@@ -1952,10 +1952,14 @@ __global__ void __launch_bounds__(BicgGridShape<T, NV>::NT, BicgGridShape<T, NV>
     __syncthreads();
 
     // partials of this chunk's pairs (operands in sa, sb), one warp per pair and
-    // column, while the last warp waits until the CTA's stores are visible
+    // column.  The threads that will store them (the last ones, a partial each)
+    // fence first, while the other warps sum: a thread's fence and its own store
+    // after it make the CTA's vector stores visible to who reads the partial.
     auto publish = [&](int nd, int c, BicgGridSlot *slots, int it) {
+        const int q0 = NT - 1 - tid;  // this thread's partial
+        const bool mine = q0 < nd * NV;
         __syncthreads();
-        if (tid == NT - 1) grid_fence();
+        if (mine) grid_fence();
         for (int q = warp; q < nd * NV; q += NT / 32) {
             const int d = q / NV, k = q % NV;
             const T *A = (d == 2 ? sb : sa) + k * PK, *B = (nd == 3 && d == 1 ? sa : sb) + k * PK;
@@ -1968,7 +1972,7 @@ __global__ void __launch_bounds__(BicgGridShape<T, NV>::NT, BicgGridShape<T, NV>
             if (wl == 0) val[q] = acc;
         }
         __syncthreads();
-        if (tid < nd * NV) slot_put(slots + (i64)tid * nch + c, val[tid], (unsigned)it);
+        if (mine) slot_put(slots + (i64)q0 * nch + c, val[q0], (unsigned)it);
     };
     // the sums over all chunks into val; false: a wait ran out
     auto collect = [&](int nd, const BicgGridSlot *slots, int it) {
