@@ -273,7 +273,11 @@ int xamg_gs_plan_error(void *plan);
 void xamg_gs_plan_destroy(void *plan);
 /* One HSGS call: t = b - A_offblock x (when hybrid), forward then backward
  * sweep updating x in place.  relax: nv values of the solver precision.
- * t_scratch: n*nv elements (needed only when block_rows > 0). */
+ * t_scratch: n*nv elements (needed only when block_rows > 0).  A plan owns
+ * synchronisation words and, for single-process sweeps, the vector between the
+ * two sweeps (allocated with the values, again by a call wider than that
+ * covers; a captured call stays valid until the plan gets other values or is
+ * destroyed), so the calls of one plan must not overlap, on any stream. */
 int xamg_hsgs(void *plan, int prec, int nv, const int *rp, const int *ci, const void *val,
               const void *invdiag, const void *b, void *x, const void *relax, void *t_scratch,
               void *stream);

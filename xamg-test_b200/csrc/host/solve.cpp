@@ -657,6 +657,23 @@ void GsPlan::build_warp(const HostCsr &A) {
     }
 }
 
+constexpr size_t kBetweenAhead = 64ull << 20;
+
+void *GsPlan::between(size_t bytes) {
+    if (wmid.empty() || wmid.back().bytes < bytes) {
+        // a wider call than any before; it may be one that is being captured
+        cudaStreamCaptureMode md = cudaStreamCaptureModeRelaxed;
+        XCUDA(cudaThreadExchangeStreamCaptureMode(&md));
+        DBuf d;
+        const cudaError_t e = cudaMalloc(&d.p, bytes);
+        cudaThreadExchangeStreamCaptureMode(&md);
+        XCUDA(e);
+        d.bytes = bytes;
+        wmid.push_back(std::move(d));
+    }
+    return wmid.back().p;
+}
+
 void GsPlan::build_lcsr(const HostCsr &A, Prec p, int nv) {
     if (mode == GsMode::LEVELS) return;
     lprec = p;
@@ -674,7 +691,13 @@ void GsPlan::build_lcsr(const HostCsr &A, Prec p, int nv) {
         // of unknown width: eight rows, a warp's of 64-byte rows
         build_items(d, nv == 0 ? 8 : xk::gs_rows_per_item(p, nv), A, p, dinv, lev, order, groups, blev);
     }
-    if (mode == GsMode::GRID && nv > 0) wmid.alloc((size_t)n * nv * prec_size(p));
+    // allocated here rather than in the first sweep: for the widest one where the
+    // width is not known, as far as that takes no more than kBetweenAhead
+    wmid.clear();
+    if (mode == GsMode::GRID && !narrow()) {
+        const size_t bytes = (size_t)n * (nv > 0 ? nv : 32) * prec_size(p);
+        between(nv > 0 ? bytes : std::min(bytes, kBetweenAhead));
+    }
     has_lcsr = true;
     lc[0].desc.release();  // the warp kernel's copy of earlier values
     if (gs_warp_sweep()) build_warp(A);
@@ -703,7 +726,7 @@ static bool warp_sweep_on() {
 
 int gs_warp_sweep() { return warp_sweep_on() ? 1 : 0; }
 
-bool GsPlan::sweeps_lcsr(Prec p, int nv, const void *t, void *x, const void *relax, cudaStream_t s) {
+void GsPlan::sweeps_lcsr(Prec p, int nv, const void *t, void *x, const void *relax, cudaStream_t s) {
     int *err = (int *)(sync.as<char>() + kSyncErrOffset);
     const Lcsr &If = lc[0], &Ib = lc[1];
     // one sweep: in-block entries (column + value), per row its id, offset
@@ -717,32 +740,25 @@ bool GsPlan::sweeps_lcsr(Prec p, int nv, const void *t, void *x, const void *rel
         KTimeScope kt(KClass::GS_WINDOW, n, 2 * gbytes, s);
         XCUDA(xk::gs_sweep_block(p, nv, nblocks, f, b, t, x, relax, brows, n, emax, err, &tile, s));
         if (tile) kt.reclass(KClass::GS_TILE);
-        return true;
+        return;
     }
     // a narrow schedule runs in one CTA of 16 warps: up to 8 items a level it
     // is the faster one (FP64, NV = 4, 27-point 32^3 hierarchy, both sweeps of a
     // level: 370 rows 386 against 726 us, 2087 rows 727 against 884, 8192 rows
     // 900 against 900, 32768 rows 1492 against 805)
-    if (If.count <= 8 * lc[0].nlev) {
+    if (narrow()) {
         bool tile = false;
         KTimeScope kt(KClass::GS_GRID, n, 2 * gbytes, s);
         XCUDA(xk::gs_sweep_block(p, nv, 1, f, b, t, x, relax, n, n, emax, err, &tile, s));
-        return true;
+        return;
     }
-    const size_t need = (size_t)n * nv * prec_size(p);
-    if (wmid.bytes < need) {
-        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-        XCUDA(cudaStreamIsCapturing(s, &st));
-        if (st != cudaStreamCaptureStatusNone) return false;
-        wmid.alloc(need);
-    }
+    void *const mid = between((size_t)n * nv * prec_size(p));
     {
         KTimeScope kt(KClass::GS_GRID, n, gbytes, s);
-        XCUDA(xk::gs_sweep_flow(p, nv, f, If.count, lc[0].nlev, 1, t, x, wmid.p, relax, n, emax, err, s));
+        XCUDA(xk::gs_sweep_flow(p, nv, f, If.count, lc[0].nlev, 1, t, x, mid, relax, n, emax, err, s));
     }
     KTimeScope kt(KClass::GS_GRID, n, gbytes, s);
-    XCUDA(xk::gs_sweep_flow(p, nv, b, Ib.count, lc[1].nlev, 0, t, wmid.p, x, relax, n, emax, err, s));
-    return true;
+    XCUDA(xk::gs_sweep_flow(p, nv, b, Ib.count, lc[1].nlev, 0, t, mid, x, relax, n, emax, err, s));
 }
 
 void GsPlan::sweeps(Prec p, int nv, const int *rp, const int *ci, const void *val, const void *invd, const void *t,
@@ -773,7 +789,8 @@ void GsPlan::sweeps(Prec p, int nv, const int *rp, const int *ci, const void *va
                 return;
             }
         }
-        if (sweeps_lcsr(p, nv, t, x, relax, s)) return;
+        sweeps_lcsr(p, nv, t, x, relax, s);
+        return;
     }
     sweep_csr(p, nv, rp, ci, val, invd, t, x, relax, true, s);
     sweep_csr(p, nv, rp, ci, val, invd, t, x, relax, false, s);

@@ -120,9 +120,13 @@ struct GsPlan {
         DBuf items, bitem, imax, scb, sva, sinvd, smeta;
         int rows = 0, count = 0, ientries = 0;  // most rows of an item, items, most entries of one
     } lc[2];
-    // GRID: the vector between the forward and the backward sweep (the plan's
-    // sweeps run one at a time)
-    DBuf wmid;
+    // GRID, schedules for the whole device: the vector between the forward and
+    // the backward sweep (the plan's sweeps run one at a time).  The last buffer
+    // is the one in use; narrower ones stay for graphs that have captured them.
+    std::vector<DBuf> wmid;
+    void *between(size_t bytes);
+    // GRID: the schedule is run by one CTA (see sweeps_lcsr)
+    bool narrow() const { return lc[0].count <= 8 * lc[0].nlev; }
     bool has_lcsr = false;
     i64 nnz_in = 0;  // entries inside the rows' blocks (all entries without blocks)
     Prec lprec = Prec::F64;
@@ -150,9 +154,8 @@ struct GsPlan {
     // forward and backward sweep
     void sweeps(Prec p, int nv, const int *rp, const int *ci, const void *val, const void *invd, const void *t,
                 void *x, const void *relax, cudaStream_t s);
-    // over the level-ordered copy by CTAs; false: not possible now (no vector
-    // between the sweeps and none may be allocated during a stream capture)
-    bool sweeps_lcsr(Prec p, int nv, const void *t, void *x, const void *relax, cudaStream_t s);
+    // over the level-ordered copy by CTAs
+    void sweeps_lcsr(Prec p, int nv, const void *t, void *x, const void *relax, cudaStream_t s);
     // one direction by the kernels that need no level-ordered copy
     void sweep_csr(Prec p, int nv, const int *rp, const int *ci, const void *val, const void *invd, const void *t,
                    void *x, const void *relax, bool forward, cudaStream_t s);
