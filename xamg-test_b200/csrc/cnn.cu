@@ -452,11 +452,13 @@ constexpr int WG_HALO = 4 * 10 * 10, WG_VOX = 128;
 template <int CO> struct WgradShape {
     static constexpr int GBYTES = (CO / 8) * WG_VOX * 16, HBYTES = 2 * WG_HALO * 16, STAGE = GBYTES + HBYTES;
 };
-template <int CO>
+// I: type of box numbers and of offsets inside a box (int, or i64 for planes or
+// counts beyond it)
+template <int CO, class I>
 __global__ void __launch_bounds__(256, CO == 64 ? 1 : 2) k_wgrad(const bf16 *__restrict__ in, int ics, int ic0, int cin,
                                                                  const bf16 *__restrict__ gr, int gcs, int gc0,
                                                                  float *dw, Vol g, int nbx, int nby, int nbz,
-                                                                 int nboxes) {
+                                                                 I nboxes) {
     typedef WgradShape<CO> S;
     extern __shared__ __align__(128) unsigned char dyn[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -466,7 +468,8 @@ __global__ void __launch_bounds__(256, CO == 64 ? 1 : 2) k_wgrad(const bf16 *__r
     // box voxel p / (CO / 8); offsets from the box's origin and, for the halo, the
     // faces it lies on
     constexpr int NH = (2 * WG_HALO + 255) / 256, NG = CO / 8 * WG_VOX / 256;
-    int ho[NH], hf[NH], go[NG];
+    int hf[NH];
+    I ho[NH], go[NG];
     auto halo_at = [&](int k, int &x, int &y, int &z) {
         const int v = (tid + 256 * k) >> 1;
         x = v % 10 - 1;
@@ -484,23 +487,23 @@ __global__ void __launch_bounds__(256, CO == 64 ? 1 : 2) k_wgrad(const bf16 *__r
     for (int k = 0; k < NH; ++k) {
         int x, y, z;
         const bool on = halo_at(k, x, y, z);
-        ho[k] = ((z * g.h + y) * g.w + x) * ics + (tid & 1) * 8;
+        ho[k] = (((I)z * g.h + y) * g.w + x) * ics + (tid & 1) * 8;
         hf[k] = on ? (x < 0) | (x == 8) << 1 | (y < 0) << 2 | (y == 8) << 3 | (z < 0) << 4 | (z == 2) << 5 : 64;
     }
 #pragma unroll
     for (int k = 0; k < NG; ++k) {
         int x, y, z;
         grad_at(k, x, y, z);
-        go[k] = ((z * g.h + y) * g.w + x) * gcs + (tid + 256 * k) % (CO / 8) * 8;
+        go[k] = (((I)z * g.h + y) * g.w + x) * gcs + (tid + 256 * k) % (CO / 8) * 8;
     }
     const bool whole = g.w % 8 == 0 && g.h % 8 == 0 && g.d % 2 == 0;
-    auto stage = [&](int box, int s) {
-        int q = box;
-        const int x0 = (q % nbx) * 8;
+    auto stage = [&](I box, int s) {
+        I q = box;
+        const int x0 = (int)(q % nbx) * 8;
         q /= nbx;
-        const int y0 = (q % nby) * 8;
+        const int y0 = (int)(q % nby) * 8;
         q /= nby;
-        const int z0 = (q % nbz) * 2;
+        const int z0 = (int)(q % nbz) * 2;
         const i64 v0 = (((i64)(q / nbz) * g.d + z0) * g.h + y0) * g.w + x0;
         unsigned char *sg = dyn + s * S::STAGE, *sh = sg + S::GBYTES + (tid & 1) * (WG_HALO * 16) + (tid >> 1) * 16;
         const bf16 *pi = in + v0 * ics + ic0 + cb, *pg = gr + v0 * gcs + gc0 + o0;
@@ -554,7 +557,8 @@ __global__ void __launch_bounds__(256, CO == 64 ? 1 : 2) k_wgrad(const bf16 *__r
         ha[j] = (unsigned)(S::GBYTES + (lane >> 4) * (WG_HALO * 16) + row * 16);
     }
     const int taps = warp < 3 ? 4 : 3;
-    int box = blockIdx.x, s = 0;
+    I box = blockIdx.x;
+    int s = 0;
     if (box < nboxes) stage(box, 0);
     for (; box < nboxes; box += gridDim.x, s ^= 1) {
         if (box + (int)gridDim.x < nboxes) stage(box + gridDim.x, s ^ 1);
@@ -566,7 +570,7 @@ __global__ void __launch_bounds__(256, CO == 64 ? 1 : 2) k_wgrad(const bf16 *__r
         // fragment is read while this one multiplies
         unsigned a[CO / 16][4], bq[2][4];
         ldm_x4_ta(bq[0], base + ha[0]);
-        const bool low = box / nbx % nby * 8 + 4 >= g.h;  // the box's rows y >= 4 lie outside: zeros
+        const bool low = (int)(box / nbx % nby) * 8 + 4 >= g.h;  // the box's rows y >= 4 lie outside: zeros
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             if ((k & 3) >= 2 && low) continue;
@@ -1203,7 +1207,7 @@ int xcnn_conv3d_wgrad(const void *in, int ics, int ic0, int cin, const void *gra
     Vol g{nb, d, h, wd};
     const int nbx = (wd + 7) / 8, nby = (h + 7) / 8, nbz = (d + 1) / 2;
     const i64 nboxes = (i64)nb * nbx * nby * nbz;
-    if (nboxes > 0x3fffffff || (i64)3 * h * wd * std::max(ics, gcs) > 0x7fffffff) return 2;  // 32-bit offsets in a box
+    const bool big = nboxes > 0x3fffffff || (i64)3 * h * wd * std::max(ics, gcs) > 0x7fffffff;
     const int co = cout > 64 ? 64 : cout, nci = cin / 16, nco = cout / co;
     // two CTAs per SM (one at 64 channels, whose partial sums fill the register
     // file), shared out over the channel chunks; every CTA has a box
@@ -1213,14 +1217,16 @@ int xcnn_conv3d_wgrad(const void *in, int ics, int ic0, int cin, const void *gra
     cudaStream_t s = (cudaStream_t)stream;
     const bf16 *pi = (const bf16 *)in;
     const bf16 *pg = (const bf16 *)grad;
-#define LW(CO)                                                                                                    \
+#define LW(CO, I)                                                                                                 \
     {                                                                                                             \
-        auto k = k_wgrad<CO>;                                                                                     \
+        auto k = k_wgrad<CO, I>;                                                                                  \
         const int sm = 2 * WgradShape<CO>::STAGE;                                                                 \
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);                                 \
-        k<<<grid, 256, sm, s>>>(pi, ics, ic0, cin, pg, gcs, gc0, dw, g, nbx, nby, nbz, (int)nboxes);              \
+        k<<<grid, 256, sm, s>>>(pi, ics, ic0, cin, pg, gcs, gc0, dw, g, nbx, nby, nbz, (I)nboxes);                \
     }
-    if (co == 16) LW(16) else if (co == 32) LW(32) else LW(64)
+#define LWI(I) { if (co == 16) LW(16, I) else if (co == 32) LW(32, I) else LW(64, I) }
+    if (big) LWI(i64) else LWI(int)
+#undef LWI
 #undef LW
     return last_err();
 }
