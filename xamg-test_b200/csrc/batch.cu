@@ -26,8 +26,9 @@ __device__ __forceinline__ int seg_of(const i64 *segoff, int nseg, i64 i) {
 
 // Stage 1 of the per-segment canonical inner products: chunks of 256 rows of
 // one segment (counted from the segment's first row), in the order and with the
-// split of the whole-vector dots (dots.cuh).
-template <class TI, int NV, int ND, bool SH>
+// split of the whole-vector dots (dots.cuh).  AL: the vectors lie on boundaries of
+// the loads (two elements); else element by element.
+template <class TI, int NV, int ND, bool SH, bool AL>
 __global__ void __launch_bounds__(256, ND == 1 ? 4 : 2) k_segdot1(int nseg, const i64 *__restrict__ segoff,
                                                  const i64 *__restrict__ cstart, i64 nch, int W,
                                                  const TI *__restrict__ a0, const TI *__restrict__ b0,
@@ -47,7 +48,7 @@ __global__ void __launch_bounds__(256, ND == 1 ? 4 : 2) k_segdot1(int nseg, cons
     if (g < nch) {
         const int s = seg_of(cstart, nseg, g);
         const i64 r0 = segoff[s] + (g - cstart[s]) * 256;
-        dot_chunk<TI, NV, ND, SH>(A, B, r0, (int)min((i64)256, segoff[s + 1] - r0), W, sub, v);
+        dot_chunk<TI, NV, ND, SH, AL>(A, B, r0, (int)min((i64)256, segoff[s + 1] - r0), W, sub, v);
     }
     if (!dot_join<NV>(W, sub, sm, v) || g >= nch) return;
     dot_fold_lanes<NV>(v);
@@ -179,13 +180,18 @@ static void segdots_t(int nseg, const i64 *segoff, const i64 *cstart, i64 nch, i
         const TI *A2 = nd > 2 ? (const TI *)a[2] : A0, *B2 = nd > 2 ? (const TI *)b[2] : B0;
         const DotSplit sp = dot_split<NV>(nch, sm_count());
         const bool sh = nd == 3 && A1 == A0 && B1 == A0 && A2 == B0 && B2 == B0;
-#define L(ND, SH)                                                                                   \
-    k_segdot1<TI, NV, ND, SH><<<sp.blocks, 32 * sp.warps, 0, s>>>(nseg, segoff, cstart, nch, sp.W, A0, B0, A1, B1, A2, \
-                                                                  B2, part)
-        if (nd == 1) L(1, false);
-        else if (nd == 2) L(2, false);
-        else if (sh) L(3, true);
-        else L(3, false);
+        uintptr_t low = 0;
+        for (int d = 0; d < nd; ++d) low |= (uintptr_t)a[d] | (uintptr_t)b[d];
+        const bool al = low % (DotShape<NV>::V * sizeof(TI)) == 0;
+#define L(ND, SH, AL)                                                                               \
+    k_segdot1<TI, NV, ND, SH, AL><<<sp.blocks, 32 * sp.warps, 0, s>>>(nseg, segoff, cstart, nch, sp.W, A0, B0, A1, B1, A2, \
+                                                                      B2, part)
+#define LA(ND) { if (al) L(ND, false, true); else L(ND, false, false); }
+        if (nd == 1) LA(1)
+        else if (nd == 2) LA(2)
+        else if (sh && al) L(3, true, true);
+        else LA(3)
+#undef LA
 #undef L
     }
     k_segdot2<<<(unsigned)(nseg * nd * NV), 256, 0, s>>>(nseg, nd * NV, NV, cstart, nch, part, out);

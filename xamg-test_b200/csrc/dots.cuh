@@ -74,9 +74,11 @@ __device__ __forceinline__ bool dot_join(int W, int sub, double *sm, double (&v)
     return true;
 }
 
-template <class TI, int V> __device__ __forceinline__ void dot_ld(const TI *p, TI (&r)[V]) {
-    if constexpr (V == 1) {
-        r[0] = __ldg(p);
+// AL: p lies on a boundary of V elements
+template <class TI, int V, bool AL> __device__ __forceinline__ void dot_ld(const TI *p, TI (&r)[V]) {
+    if constexpr (V == 1 || !AL) {
+#pragma unroll
+        for (int e = 0; e < V; ++e) r[e] = __ldg(p + e);
     } else if constexpr (sizeof(TI) == 8) {
         const double2 w = __ldg(reinterpret_cast<const double2 *>(p));
         r[0] = w.x, r[1] = w.y;
@@ -88,7 +90,7 @@ template <class TI, int V> __device__ __forceinline__ void dot_ld(const TI *p, T
 
 // This thread's part of ND pairs over the cnt <= 256 rows from row0, the subtree
 // `sub` of W.  SH: the pairs are (a, b), (a, a), (b, b) of two vectors.
-template <class TI, int NV, int ND, bool SH>
+template <class TI, int NV, int ND, bool SH, bool AL = true>
 __device__ __forceinline__ void dot_chunk(const TI *const (&A)[ND], const TI *const (&B)[ND], i64 row0, int cnt, int W,
                                           int sub, double (&out)[ND * DotShape<NV>::V]) {
     typedef DotShape<NV> S;
@@ -110,8 +112,8 @@ __device__ __forceinline__ void dot_chunk(const TI *const (&A)[ND], const TI *co
                 for (int u = 0; u < U; ++u)
 #pragma unroll
                     for (int d = 0; d < (SH ? 1 : ND); ++d) {
-                        dot_ld<TI, V>(A[d] + o + (m + u) * 32 * NV, a[u][d]);
-                        dot_ld<TI, V>(B[d] + o + (m + u) * 32 * NV, b[u][d]);
+                        dot_ld<TI, V, AL>(A[d] + o + (m + u) * 32 * NV, a[u][d]);
+                        dot_ld<TI, V, AL>(B[d] + o + (m + u) * 32 * NV, b[u][d]);
                     }
 #pragma unroll
                 for (int u = 0; u < U; ++u)
@@ -129,8 +131,8 @@ __device__ __forceinline__ void dot_chunk(const TI *const (&A)[ND], const TI *co
 #pragma unroll
                 for (int d = 0; d < ND; ++d) {
                     TI a[V], b[V];
-                    dot_ld<TI, V>(A[d] + o + m * 32 * NV, a);
-                    dot_ld<TI, V>(B[d] + o + m * 32 * NV, b);
+                    dot_ld<TI, V, AL>(A[d] + o + m * 32 * NV, a);
+                    dot_ld<TI, V, AL>(B[d] + o + m * 32 * NV, b);
 #pragma unroll
                     for (int e = 0; e < V; ++e) out[d * V + e] = fma((double)a[e], (double)b[e], out[d * V + e]);
                 }
