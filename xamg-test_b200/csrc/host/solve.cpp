@@ -452,8 +452,10 @@ static void upload_values(DBuf &dst, const std::vector<double> &v, Prec p) {
 // Cut the level-ordered rows of one direction into items of at most `rows` rows
 // of one level and gs_item_entries entries (a longer row alone); see xk::GsDir
 // for the layout.  The rows of a level are independent, so they are taken
-// longest first: an item's rows then have about the same length.
-void GsPlan::build_items(int d, int rows, const HostCsr &A, Prec p, const std::vector<double> &dinv,
+// longest first: an item's rows then have about the same length.  false: a row
+// has more groups than an item can name (2^16), or the copy more than 2^31
+// entries.
+bool GsPlan::build_items(int d, int rows, const HostCsr &A, Prec p, const std::vector<double> &dinv,
                          const std::vector<int> &lev, const std::vector<int> &order, const std::vector<int> &groups,
                          const std::vector<int> &blev) {
     Lcsr &L = lc[d];
@@ -500,8 +502,7 @@ void GsPlan::build_items(int d, int rows, const HostCsr &A, Prec p, const std::v
                 while (z < lr.size() && (int)(z - s) < rows && 4 * ng * (int)(z - s + 1) <= cap) ++z;
                 const int R = (int)(z - s), ne = 4 * ng * R;
                 const int e0 = (int)sci.size(), r0 = (int)(meta.size() / 4);
-                XCHECK((i64)sci.size() + ne < (1ll << 31) - 8, "level-ordered matrix too large");
-                XCHECK(ng < 65536, "row too long for the level-ordered copy");
+                if (ng >= 65536 || (i64)sci.size() + ne >= (1ll << 31) - 8) return false;
                 sci.resize(sci.size() + ne, pad);
                 sva.resize(sva.size() + ne, 0.0);
                 int k0 = ng;
@@ -551,6 +552,7 @@ void GsPlan::build_items(int d, int rows, const HostCsr &A, Prec p, const std::v
     upload_ints(L.scb, sci);
     upload_values(L.sva, sva, p);
     upload_values(L.sinvd, sinvd, p);
+    return true;
 }
 
 xk::GsDir GsPlan::dir(int d) const {
@@ -677,6 +679,9 @@ void *GsPlan::between(size_t bytes) {
 void GsPlan::build_lcsr(const HostCsr &A, Prec p, int nv) {
     if (mode == GsMode::LEVELS) return;
     lprec = p;
+    has_lcsr = false;
+    lc[0].desc.release();  // the warp kernel's copy of earlier values
+    wmid.clear();
     const std::vector<double> dinv = inverse_diagonal(A, p);
     nnz_in = 0;
     for (i64 i = 0; i < n; ++i) {
@@ -689,17 +694,16 @@ void GsPlan::build_lcsr(const HostCsr &A, Prec p, int nv) {
         schedule(d, order, groups, blev);
         lc[d].nlev = (int)groups.size() - 1;
         // of unknown width: eight rows, a warp's of 64-byte rows
-        build_items(d, nv == 0 ? 8 : xk::gs_rows_per_item(p, nv), A, p, dinv, lev, order, groups, blev);
+        // without the copy the sweeps run over the matrix as given (sweep_csr)
+        if (!build_items(d, nv == 0 ? 8 : xk::gs_rows_per_item(p, nv), A, p, dinv, lev, order, groups, blev)) return;
     }
     // allocated here rather than in the first sweep: for the widest one where the
     // width is not known, as far as that takes no more than kBetweenAhead
-    wmid.clear();
     if (mode == GsMode::GRID && !narrow()) {
         const size_t bytes = (size_t)n * (nv > 0 ? nv : 32) * prec_size(p);
         between(nv > 0 ? bytes : std::min(bytes, kBetweenAhead));
     }
     has_lcsr = true;
-    lc[0].desc.release();  // the warp kernel's copy of earlier values
     if (gs_warp_sweep()) build_warp(A);
 }
 

@@ -141,7 +141,7 @@ struct GsPlan {
     void build_lcsr(const HostCsr &A, Prec p, int nv);
     void build_offblock(const HostCsr &A, Prec p);
     // gs.cu's copy of one sweep direction (called by build_lcsr)
-    void build_items(int d, int rows, const HostCsr &A, Prec p, const std::vector<double> &dinv,
+    bool build_items(int d, int rows, const HostCsr &A, Prec p, const std::vector<double> &dinv,
                      const std::vector<int> &lev, const std::vector<int> &order, const std::vector<int> &groups,
                      const std::vector<int> &blev);
     xk::GsDir dir(int d) const;
