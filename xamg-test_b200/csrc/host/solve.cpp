@@ -542,6 +542,7 @@ bool GsPlan::build_items(int d, int rows, const HostCsr &A, Prec p, const std::v
         bitem.push_back((int)(items.size() / 4));
     }
     L.count = (int)(items.size() / 4);
+    L.widest = *std::max_element(imax.begin(), imax.end());
     if (items.empty()) items.assign(4, 0);
     if (meta.empty()) meta.assign(4, 0), sinvd.assign(1, 0.0);
     if (sci.empty()) sci.assign(8, pad), sva.assign(8, 0.0);
@@ -730,6 +731,10 @@ static bool warp_sweep_on() {
 
 int gs_warp_sweep() { return warp_sweep_on() ? 1 : 0; }
 
+bool GsPlan::block_arrivals_fit(Prec p, int nv) const {
+    return xk::gs_block_arrivals_fit(p, nv, lc[0].rows, std::max(lc[0].widest, lc[1].widest));
+}
+
 void GsPlan::sweeps_lcsr(Prec p, int nv, const void *t, void *x, const void *relax, cudaStream_t s) {
     int *err = (int *)(sync.as<char>() + kSyncErrOffset);
     const Lcsr &If = lc[0], &Ib = lc[1];
@@ -750,7 +755,7 @@ void GsPlan::sweeps_lcsr(Prec p, int nv, const void *t, void *x, const void *rel
     // is the faster one (FP64, NV = 4, 27-point 32^3 hierarchy, both sweeps of a
     // level: 370 rows 386 against 726 us, 2087 rows 727 against 884, 8192 rows
     // 900 against 900, 32768 rows 1492 against 805)
-    if (narrow()) {
+    if (narrow() && block_arrivals_fit(p, nv)) {
         bool tile = false;
         KTimeScope kt(KClass::GS_GRID, n, 2 * gbytes, s);
         XCUDA(xk::gs_sweep_block(p, nv, 1, f, b, t, x, relax, n, n, emax, err, &tile, s));
@@ -793,8 +798,10 @@ void GsPlan::sweeps(Prec p, int nv, const int *rp, const int *ci, const void *va
                 return;
             }
         }
-        sweeps_lcsr(p, nv, t, x, relax, s);
-        return;
+        if (mode != GsMode::BLOCKS || block_arrivals_fit(p, nv)) {
+            sweeps_lcsr(p, nv, t, x, relax, s);
+            return;
+        }
     }
     sweep_csr(p, nv, rp, ci, val, invd, t, x, relax, true, s);
     sweep_csr(p, nv, rp, ci, val, invd, t, x, relax, false, s);

@@ -119,6 +119,7 @@ struct GsPlan {
         // gs.cu's copy: items of a few rows (see xk::GsDir)
         DBuf items, bitem, imax, scb, sva, sinvd, smeta;
         int rows = 0, count = 0, ientries = 0;  // most rows of an item, items, most entries of one
+        int widest = 0;                         // most items of a level (of one block)
     } lc[2];
     // GRID, schedules for the whole device: the vector between the forward and
     // the backward sweep (the plan's sweeps run one at a time).  The last buffer
@@ -154,6 +155,8 @@ struct GsPlan {
     // forward and backward sweep
     void sweeps(Prec p, int nv, const int *rp, const int *ci, const void *val, const void *invd, const void *t,
                 void *x, const void *relax, cudaStream_t s);
+    // whether a level's items can arrive at one barrier (the block kernel)
+    bool block_arrivals_fit(Prec p, int nv) const;
     // over the level-ordered copy by CTAs
     void sweeps_lcsr(Prec p, int nv, const void *t, void *x, const void *relax, cudaStream_t s);
     // one direction by the kernels that need no level-ordered copy
