@@ -678,9 +678,7 @@ static int item_split(int rows, int rpw) {
     return s;
 }
 
-bool gs_block_arrivals_fit(Prec p, int nv, int rows, int widest) {
-    return ((i64)widest << item_split(rows, gs_rows_per_item(p, nv))) < (1 << 20);
-}
+int gs_item_warps(Prec p, int nv, int rows) { return 1 << item_split(rows, gs_rows_per_item(p, nv)); }
 
 template <class T, int NV, bool XS, int NT>
 static cudaError_t gs_block_l(int nblocks, const GsDir &f, const GsDir &b, const T *t, T *x, const T *relax, int brows,

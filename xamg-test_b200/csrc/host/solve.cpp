@@ -700,7 +700,7 @@ void GsPlan::build_lcsr(const HostCsr &A, Prec p, int nv) {
     }
     // allocated here rather than in the first sweep: for the widest one where the
     // width is not known, as far as that takes no more than kBetweenAhead
-    if (mode == GsMode::GRID && !narrow()) {
+    if (mode == GsMode::GRID && !narrow(p, nv > 0 ? nv : 32)) {
         const size_t bytes = (size_t)n * (nv > 0 ? nv : 32) * prec_size(p);
         between(nv > 0 ? bytes : std::min(bytes, kBetweenAhead));
     }
@@ -732,7 +732,17 @@ static bool warp_sweep_on() {
 int gs_warp_sweep() { return warp_sweep_on() ? 1 : 0; }
 
 bool GsPlan::block_arrivals_fit(Prec p, int nv) const {
-    return xk::gs_block_arrivals_fit(p, nv, lc[0].rows, std::max(lc[0].widest, lc[1].widest));
+    return (i64)std::max(lc[0].widest, lc[1].widest) * xk::gs_item_warps(p, nv, lc[0].rows) < (1 << 20);
+}
+
+// Up to 8 warps' shares a level one CTA is the faster one (both sweeps of a call,
+// us, one CTA / whole device, by shares a level: 27-point FP64 NV 8 3.3 134 / 265,
+// 5.1 283 / 361, 7.9 513 / 447, 11 896 / 541; FP32 NV 4 7.9 379 / 478, 11 820 / 573;
+// FP64 NV 1 7.9 305 / 443, 11 535 / 550, 15 922 / 659; 7-point FP64 NV 8 6.8 52 / 60,
+// 11.6 126 / 79).  Shares, not items: at FP64 NV 32 an item of eight rows takes four
+// warps (27-point 20^3, 8 items and 32 shares a level: 1619 / 433).
+bool GsPlan::narrow(Prec p, int nv) const {
+    return (i64)lc[0].count * xk::gs_item_warps(p, nv, lc[0].rows) <= 8ll * lc[0].nlev;
 }
 
 void GsPlan::sweeps_lcsr(Prec p, int nv, const void *t, void *x, const void *relax, cudaStream_t s) {
@@ -751,11 +761,8 @@ void GsPlan::sweeps_lcsr(Prec p, int nv, const void *t, void *x, const void *rel
         if (tile) kt.reclass(KClass::GS_TILE);
         return;
     }
-    // a narrow schedule runs in one CTA of 16 warps: up to 8 items a level it
-    // is the faster one (FP64, NV = 4, 27-point 32^3 hierarchy, both sweeps of a
-    // level: 370 rows 386 against 726 us, 2087 rows 727 against 884, 8192 rows
-    // 900 against 900, 32768 rows 1492 against 805)
-    if (narrow() && block_arrivals_fit(p, nv)) {
+    // a narrow schedule runs in one CTA of 16 warps
+    if (narrow(p, nv) && block_arrivals_fit(p, nv)) {
         bool tile = false;
         KTimeScope kt(KClass::GS_GRID, n, 2 * gbytes, s);
         XCUDA(xk::gs_sweep_block(p, nv, 1, f, b, t, x, relax, n, n, emax, err, &tile, s));

@@ -127,7 +127,7 @@ struct GsPlan {
     std::vector<DBuf> wmid;
     void *between(size_t bytes);
     // GRID: the schedule is run by one CTA (see sweeps_lcsr)
-    bool narrow() const { return lc[0].count <= 8 * lc[0].nlev; }
+    bool narrow(Prec p, int nv) const;
     bool has_lcsr = false;
     i64 nnz_in = 0;  // entries inside the rows' blocks (all entries without blocks)
     Prec lprec = Prec::F64;

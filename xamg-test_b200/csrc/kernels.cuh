@@ -114,13 +114,13 @@ constexpr unsigned long long kGsWaitNs = 1000000000ull;  // 1 s
 // single row may have more)
 int gs_rows_per_item(Prec p, int nv);
 int gs_item_entries();
-// whether the `widest` items of a level, of at most `rows` rows each, are arrivals
-// that an mbarrier can count (2^20 - 1): a condition of gs_sweep_block
-bool gs_block_arrivals_fit(Prec p, int nv, int rows, int widest);
+// warps that an item of at most `rows` rows is shared out to (nv columns)
+int gs_item_warps(Prec p, int nv, int rows);
 // Forward and backward sweep of every block in one launch, one CTA per block
 // (512 threads when there is at most one block per SM, 256 with two, else 128).
 // emax: the most entries of one item.  *tile: whether the x tile was in shared
-// memory.  A wait that takes longer than limit_ns sets *err.
+// memory.  A level's items times their warps are arrivals at an mbarrier: at most
+// 2^20 - 1.  A wait that takes longer than limit_ns sets *err.
 cudaError_t gs_sweep_block(Prec p, int nv, int nblocks, const GsDir &f, const GsDir &b, const void *t, void *x,
                            const void *relax, i64 brows, i64 n, int emax, int *err, bool *tile, cudaStream_t s,
                            unsigned long long limit_ns = kGsWaitNs);
