@@ -1108,30 +1108,42 @@ int last_err() {
 bool box_weights_resident(int bn, int kc) { return bn < 64 && kc * 27 * bn * 32 <= 56 * 1024; }
 
 // Output channels and depth of the box kernel's CTAs: the pair with the least
-// estimated time.  A tap of one warp takes bn cycles of the SM's tensor pipe and
-// 16 + bn / 4 of its shared memory, of which about a quarter overlap (measured:
-// 48 -> 16 channels at 8 x 64^3), and no less than the latency of its reads and
-// mma; every chunk is copied by the CTA's own threads.  Wide CTAs read less, narrow ones leave more warps on a small volume
-// (8 x 16^3, 64 -> 64: bn 64 58 us, 16 43 us; 8 x 8^3, 128 -> 128: 55 and 25 us).
+// estimated time (SM cycles).  A round is a box of every CTA that fits; its chunk
+// takes 27 taps, each no less than the latency of its reads and mma and no less
+// than the resident warps' tensor and shared-memory cycles, and the issue of its
+// copies: 48 cycles a 16-byte halo piece and 31 a weight piece of a thread, or 40
+// and 91 divided among the warps of a scheduler.  All CTAs' copies share the L2 (70
+// bytes a cycle and SM); resident weights are copied once.  The numbers minimise
+// the loss of the choice over 804 layers (10 channel pairs, 3^3 to 40^3, 1 to 8
+// volumes, all pairs timed): it is on average 1 % from the best pair.  The estimate
+// before did not see that a small CTA has as many weights to copy as a large one:
+// 3 x 24^3, 64 -> 64 took 63 us (bn 32, bz 2), now 49; 5 x 16^3, 128 -> 128 117 and 92;
+// 6 x 24^3, 96 -> 32 86 and 60; 8 x 20^3, 16 -> 32 20.4 and 15.9.
 struct BoxPlan {
     int bn, bz;
-    double t;  // SM cycles
+    double t;
 };
 BoxPlan box_plan(i64 plane, int d, int kc, int cout, int bn0) {
     BoxPlan best{bn0, 8, 1e300};
+    const int sms = xk::sm_count();
     for (int bn = bn0; bn >= 16; bn /= 2)
         for (int bz = 8; bz >= 2; bz /= 2) {
             const i64 tasks = plane * ((d + bz - 1) / bz) * (cout / bn);
+            const bool res = box_weights_resident(bn, kc);
             const int halo = (bz + 2) * 100 * 32, wb = 27 * bn * 32;
-            const int sm = box_weights_resident(bn, kc) ? 2 * halo + kc * wb : 2 * (halo + wb);
+            const int sm = res ? 2 * halo + kc * wb : 2 * (halo + wb);
             const i64 fit = std::max(1, std::min(227 * 1024 / (sm + 2048), (bn == 16 ? 16 : 8) / bz));
-            const i64 rounds = (tasks + 148 * fit - 1) / (148 * fit);
-            const double warps = (double)std::min<i64>(fit, (tasks + 147) / 148) * bz;
-            const double tap = std::max(60.0 + 2.2 * bn, 0.75 * warps * (1.25 * bn + 16));
+            const i64 rounds = (tasks + sms * fit - 1) / (sms * fit);
+            const double warps = (double)std::min<i64>(fit, (tasks + sms - 1) / sms) * bz;
+            const double tap = std::max(14.0 + 2.0 * bn, 0.8 * warps * (0.79 * bn + 6.5));
+            const double pieces = 1.0 / 16 / (32 * bz);  // of a thread, per byte
+            const double copy = 260.0 + pieces * (halo * std::max(48.0, 40.0 / 4 * warps) +
+                                                  (res ? 0.0 : wb * std::max(31.0, 91.0 / 4 * warps)));
             // a lone CTA on its SM has nobody to compute while it stages
-            const double copy = 500.0 + 20.0 / 16 * (halo + (box_weights_resident(bn, kc) ? 0 : wb)) / (32 * bz);
-            const double t = (double)rounds * kc * (27 * tap + copy) * (fit == 1 ? 1.25 : 1.0);
-            if (t < best.t * 0.98) best = {bn, bz, t};
+            double t = (double)rounds * kc * (27 * tap + copy) * (fit == 1 ? 1.26 : 1.0) + 1100.0;
+            t += 0.014 / sms * (double)tasks * kc * (halo + (res ? 0 : wb));
+            if (res) t += 110.0 * pieces * kc * wb;
+            if (t < best.t * 0.95) best = {bn, bz, t};
         }
     return best;
 }
@@ -1162,14 +1174,14 @@ int xcnn_conv3d(const void *in, int ics, int ic0, int cin, const void *w, const 
         return last_err();
     }
     // box kernel unless padding the volume to boxes costs more than the
-    // voxel-tile kernel's steps (one per tap and chunk, about 700 cycles each
+    // voxel-tile kernel's steps (one per tap and chunk, about 1300 cycles each
     // while its tiles fill an SM up to three times)
     auto up = [](int n, int m) { return (n + m - 1) / m; };
     const i64 plane = (i64)nb * up(h, 8) * up(wd, 8);
     const BoxPlan bp = box_plan(plane, d, cin / 16, cout, bn0);
     const int bn = bp.bn, bz = bp.bz;
     const i64 nboxes = plane * up(d, bz), tiles = (nvox + BM - 1) / BM * (cout / bn0);
-    if (box_conv_enabled() && nboxes <= 0x3fffffff && bp.t < 27.0 * (cin / 16) * 700.0 * (double)((tiles + 443) / 444) &&
+    if (box_conv_enabled() && nboxes <= 0x3fffffff && bp.t < 27.0 * (cin / 16) * 1300.0 * (double)((tiles + 3 * xk::sm_count() - 1) / (3 * xk::sm_count())) &&
         (i64)10 * h * wd * ics <= 0x7fffffff && (i64)wd * ocs <= 0x7fffffff) {
 #define LB(BN, BZ, WRES)                                                                                            \
     {                                                                                                               \

@@ -19,8 +19,6 @@
 
 namespace xk {
 
-int sm_count();  // of the current device
-
 template <int NV> struct DotShape {
     static constexpr int V = NV == 1 ? 1 : 2, TPR = NV / V, RPI = 32 / TPR;
     static constexpr int LOG = TPR == 1 ? 0 : TPR == 2 ? 1 : TPR == 4 ? 2 : TPR == 8 ? 3 : 4;

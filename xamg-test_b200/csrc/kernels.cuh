@@ -22,6 +22,7 @@ enum class Prec : int { F64 = 0, F32 = 1 };
 // Count of kernels this library has launched (every launcher adds its own).
 void note_launch(int k = 1);
 long long launch_count();
+int sm_count();  // of the device of the process's first call
 
 // ---- sparse matrix-vector products ---------------------------------------
 // y = A x (mode 0), y += A x (mode 1), y = b - A x (mode 2, b given).
