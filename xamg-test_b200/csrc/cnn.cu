@@ -1091,7 +1091,8 @@ bool box_conv_enabled() { return g_box_conv != 0; }
 
 int grid_for(i64 n) {
     i64 g = (n + 255) / 256;
-    return (int)(g < 148 * 16 ? (g < 1 ? 1 : g) : 148 * 16);
+    const i64 most = xk::sm_count() * 16;
+    return (int)(g < most ? (g < 1 ? 1 : g) : most);
 }
 
 int last_err() {
@@ -1191,7 +1192,7 @@ int xcnn_conv3d(const void *in, int ics, int ic0, int cin, const void *w, const 
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);                                   \
         int per = 0;                                                                                                \
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, S::NT, sm) != cudaSuccess || per < 1) per = 1;    \
-        dim3 gb((unsigned)std::max<i64>(1, std::min<i64>(nboxes, (i64)148 * per / (cout / bn))), (unsigned)(cout / bn)); \
+        dim3 gb((unsigned)std::max<i64>(1, std::min<i64>(nboxes, (i64)xk::sm_count() * per / (cout / bn))), (unsigned)(cout / bn)); \
         k<<<gb, S::NT, sm, s>>>(pi, ics, ic0, cin, pw, bias, po, ocs, oc0, g, up(wd, 8), up(h, 8), up(d, bz), (int)nboxes, flags); \
     }
 #define LBZ(BN, WRES)                                                                                               \
@@ -1223,7 +1224,7 @@ int xcnn_conv3d_wgrad(const void *in, int ics, int ic0, int cin, const void *gra
     const int co = cout > 64 ? 64 : cout, nci = cin / 16, nco = cout / co;
     // two CTAs per SM (one at 64 channels, whose partial sums fill the register
     // file), shared out over the channel chunks; every CTA has a box
-    const i64 want = (i64)148 * (co == 64 ? 1 : 2) / (nci * nco);
+    const i64 want = (i64)xk::sm_count() * (co == 64 ? 1 : 2) / (nci * nco);
     const unsigned slices = (unsigned)std::max<i64>(0, want < 1 ? std::min<i64>(1, nboxes) : std::min(want, nboxes));
     dim3 grid(slices, (unsigned)nci, (unsigned)nco);
     cudaStream_t s = (cudaStream_t)stream;
@@ -1265,7 +1266,7 @@ int xcnn_bias_grad(const void *g, int gcs, int gc0, int c, int64_t nvox, float *
     if (c % 8 == 0 && gcs % 8 == 0 && gc0 % 8 == 0 && (uintptr_t)g % 16 == 0 && nvox > 0) {
         // slices of about 64 voxels a thread row, at most four blocks per SM
         const i64 rows = 256 / (c / 8);
-        const i64 blocks = std::min<i64>(148 * 4, (nvox + rows * 16 - 1) / (rows * 16));
+        const i64 blocks = std::min<i64>(xk::sm_count() * 4, (nvox + rows * 16 - 1) / (rows * 16));
         const i64 slice = (nvox + blocks - 1) / blocks;
         k_bias_grad<<<(unsigned)((nvox + slice - 1) / slice), 256, 0, s>>>((const bf16 *)g, gcs, gc0, c / 8, nvox, slice, db);
         return last_err();
