@@ -798,7 +798,7 @@ int xamg_spmv_runs_plan_info(void *plan, int64_t *nchunks, double *coverage, int
             for (i64 c = 0; c < h->nchunks; ++c) s += h->hchunks[(size_t)c * 4 + 3];
             *segments = s;
         }
-        if (value_slots) *value_slots = h->hvoff.empty() ? 0 : h->hvoff.back() * h->R;
+        if (value_slots) *value_slots = h->slots();
     });
 }
 int xamg_spmv_runs(void *plan, int prec, int nv, const void *x, void *y, int mode, const void *b, void *stream) {
@@ -810,7 +810,7 @@ int xamg_spmv_runs(void *plan, int prec, int nv, const void *x, void *y, int mod
         XCHECK(mode != 2 || b, "mode 2 needs b");
         XCHECK(xk::spmv_runs_supported((Prec)prec, nv), "shape not supported (FP64 nv 8, 16, 32; FP32 nv 16, 32)");
         XCHECK(h->has((Prec)prec), "plan has no values in this precision");
-        xk::spmv_runs((Prec)prec, nv, h->nchunks, h->ntiles, h->chunks.as<int4>(), h->toff.as<longlong2>(),
+        xk::spmv_runs((Prec)prec, nv, h->n, h->slots(), h->nchunks, h->ntiles, h->chunks.as<int4>(), h->toff.as<longlong2>(),
                       h->sg.as<int>(), prec == 0 ? h->v64.p : h->v32.p, x, y, mode, b, strm(stream));
         XCUDA(cudaGetLastError());
     });

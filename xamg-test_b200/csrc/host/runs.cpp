@@ -12,7 +12,7 @@ namespace xamg {
 
 void RunPlan::clear() {
     R = 0;
-    nchunks = ntiles = nseg = 0;
+    n = nchunks = ntiles = nseg = 0;
     coverage = 0.0;
     hchunks.clear();
     hvoff.clear();
@@ -100,6 +100,7 @@ bool RunPlan::build(const HostCsr &h, int R_, bool f64, bool f32, double min_cov
         return false;
     }
     R = R_;
+    n = h.n;
     nchunks = (i64)ch.size() / 4;
     while (ch.size() % 16) ch.insert(ch.end(), {0, 0, 0, 0});  // whole tiles of four chunks
     ntiles = (i64)ch.size() / 16;
@@ -184,7 +185,7 @@ void DCsr::spmv(Prec p, int nv, const void *x, void *y, int mode, const void *b,
         // run format: values once, 4 B per segment, 20 B per chunk (descriptor
         // and its share of the tile offsets)
         KTimeScope kt(KClass::SPMV, n, (double)nnz * sv + 4.0 * runs.nseg + 20.0 * runs.nchunks + xy, s);
-        xk::spmv_runs(p, nv, runs.nchunks, runs.ntiles, runs.chunks.as<int4>(), runs.toff.as<longlong2>(),
+        xk::spmv_runs(p, nv, n, runs.slots(), runs.nchunks, runs.ntiles, runs.chunks.as<int4>(), runs.toff.as<longlong2>(),
                       runs.sg.as<int>(), p == Prec::F64 ? runs.v64.p : runs.v32.p, x, y, mode, b, s);
         return;
     }

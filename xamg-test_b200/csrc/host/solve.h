@@ -39,7 +39,7 @@ struct DVec {
 // the row offset, with the values reordered entry-major per chunk.
 struct RunPlan {
     int R = 0;
-    i64 nchunks = 0, ntiles = 0, nseg = 0;
+    i64 n = 0, nchunks = 0, ntiles = 0, nseg = 0;
     double coverage = 0.0;     // fraction of the entries that lie in chunks of R rows
     std::vector<int> hchunks;  // {r0, cnt, m, segments} per chunk (host)
     std::vector<i64> hvoff;    // per tile of four chunks: first value slot (host, ntiles + 1)
@@ -48,6 +48,7 @@ struct RunPlan {
     // least min_cov of the entries lie in chunks of R rows, else clears it.
     bool build(const HostCsr &h, int R_, bool f64, bool f32, double min_cov);
     void add_values(const HostCsr &h, Prec p);  // values of another precision
+    i64 slots() const { return hvoff.empty() ? 0 : hvoff.back() * R; }  // values, padding included
     bool has(Prec p) const { return nchunks > 0 && (p == Prec::F64 ? v64.p != nullptr : v32.p != nullptr); }
     void clear();
 };

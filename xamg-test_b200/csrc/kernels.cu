@@ -578,11 +578,9 @@ __device__ __forceinline__ void run_rows(const int4 cd, int smax, const int *sg,
         for (int q = 0; q < R; ++q)
             if (q < cd.y) ld<T, V>(y + ((i64)cd.x + q) * NV + l * V, acc[q]);
     }
-    if (MODE == 2 && NV * sizeof(T) >= 128) {
-        // b is wanted after the last segment, when there is nothing left to hide its
-        // latency behind: its lines are asked for now (27-point 64^3, us before and
-        // after: FP64 NV 16 69.4 and 64.9, NV 32 108.1 and 97.9, FP32 NV 32 61.7 and
-        // 56.9; rows of 64 bytes gain nothing, FP32 NV 16 29.9 and 30.7)
+    if (MODE == 3) {
+        // mode 2 of large vectors: b is wanted after the last segment, when there is
+        // nothing left to hide its latency behind; its lines are asked for now
         const char *line = reinterpret_cast<const char *>(b + (i64)cd.x * NV);
         for (int o = l * 128; o < cd.y * NV * (int)sizeof(T); o += Shape<T, NV>::TPR * 128)
             asm volatile("prefetch.global.L1 [%0];" ::"l"(line + o));
@@ -658,7 +656,7 @@ __device__ __forceinline__ void run_rows(const int4 cd, int smax, const int *sg,
     for (int q = 0; q < R; ++q) {
         if (q >= cd.y) break;
         const i64 row = (i64)cd.x + q;
-        if (MODE == 2) {
+        if (MODE >= 2) {
             T bb[V];
             ld<T, V>(b + row * NV + l * V, bb);
 #pragma unroll
@@ -730,7 +728,7 @@ bool spmv_runs_supported(Prec p, int nv) {
 }
 
 template <class T, int NV, int NT, bool STX>
-static void spmv_runs_p(i64 nchunks, i64 ntiles, const int4 *chunks, const longlong2 *toff, const int *sg,
+static void spmv_runs_p(i64 n, i64 slots, i64 nchunks, i64 ntiles, const int4 *chunks, const longlong2 *toff, const int *sg,
                         const T *vt, const T *x, T *y, int mode, const T *b, cudaStream_t s) {
     typedef RunShape<T, NV, NT> RS;
     constexpr int SM = RS::SMEM_BYTES + (STX ? RunXs<NT>::BYTES : 0);
@@ -739,6 +737,8 @@ static void spmv_runs_p(i64 nchunks, i64 ntiles, const int4 *chunks, const longl
         cudaFuncSetAttribute(k_spmv_runs<T, NV, 0, NT, STX>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM);
         cudaFuncSetAttribute(k_spmv_runs<T, NV, 1, NT, STX>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM);
         cudaFuncSetAttribute(k_spmv_runs<T, NV, 2, NT, STX>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM);
+        if constexpr (NV * sizeof(T) >= 128)
+            cudaFuncSetAttribute(k_spmv_runs<T, NV, 3, NT, STX>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM);
         attr = true;
     }
     unsigned g = (unsigned)((ntiles + RS::TPC - 1) / RS::TPC);
@@ -746,29 +746,42 @@ static void spmv_runs_p(i64 nchunks, i64 ntiles, const int4 *chunks, const longl
         k_spmv_runs<T, NV, 0, NT, STX><<<g, NT, SM, s>>>(nchunks, ntiles, chunks, toff, sg, vt, x, y, b);
     else if (mode == 1)
         k_spmv_runs<T, NV, 1, NT, STX><<<g, NT, SM, s>>>(nchunks, ntiles, chunks, toff, sg, vt, x, y, b);
-    else
+    else {
+        // b's lines ahead where the three vectors and the values no longer stay in L2
+        // (us without and with: 7-point 64^3 FP64 NV 16 48.0 and 42.6, NV 32 79.5 and
+        // 68.9, FP32 NV 32 46.2 and 40.7, 27-point 69.0 and 64.1, 107.5 and 97.4, 62.4 and
+        // 56.8).  Below that it costs 1 to 3 %; the line, in MB: 7-point 56^3 FP32 NV 32
+        // (72) 23.3 and 24.2, FP64 NV 16 (77) 25.7 and 25.7, 46^3 FP64 NV 32 (80) 30.0 and
+        // 29.1, 27-point 50^3 FP64 NV 16 (75) 29.7 and 29.7, 56^3 (105) 52.1 and 49.1.  Rows
+        // of 64 bytes gain nothing (27-point 64^3 FP32 NV 16 29.9 and 30.7).
+        if constexpr (NV * sizeof(T) >= 128)
+            if ((3 * n * NV + slots) * (i64)sizeof(T) >= 80000000) {
+                k_spmv_runs<T, NV, 3, NT, STX><<<g, NT, SM, s>>>(nchunks, ntiles, chunks, toff, sg, vt, x, y, b);
+                return;
+            }
         k_spmv_runs<T, NV, 2, NT, STX><<<g, NT, SM, s>>>(nchunks, ntiles, chunks, toff, sg, vt, x, y, b);
+    }
 }
 
 template <class T, int NV>
-static void spmv_runs_t(i64 nchunks, i64 ntiles, const int4 *chunks, const longlong2 *toff, const int *sg,
+static void spmv_runs_t(i64 n, i64 slots, i64 nchunks, i64 ntiles, const int4 *chunks, const longlong2 *toff, const int *sg,
                         const T *vt, const T *x, T *y, int mode, const T *b, cudaStream_t s) {
     if constexpr (NV >= 8 && NV * sizeof(T) >= 64) {
         if (nchunks <= 0) return;
         note_launch();
-        if (g_run_form) spmv_runs_p<T, NV, RUN_NT, true>(nchunks, ntiles, chunks, toff, sg, vt, x, y, mode, b, s);
-        else spmv_runs_p<T, NV, RUN_NT, false>(nchunks, ntiles, chunks, toff, sg, vt, x, y, mode, b, s);
+        if (g_run_form) spmv_runs_p<T, NV, RUN_NT, true>(n, slots, nchunks, ntiles, chunks, toff, sg, vt, x, y, mode, b, s);
+        else spmv_runs_p<T, NV, RUN_NT, false>(n, slots, nchunks, ntiles, chunks, toff, sg, vt, x, y, mode, b, s);
     }
 }
 
-void spmv_runs(Prec p, int nv, i64 nchunks, i64 ntiles, const int4 *chunks, const longlong2 *toff, const int *sg,
+void spmv_runs(Prec p, int nv, i64 n, i64 slots, i64 nchunks, i64 ntiles, const int4 *chunks, const longlong2 *toff, const int *sg,
                const void *vt, const void *x, void *y, int mode, const void *b, cudaStream_t s) {
     if (p == Prec::F64) {
-#define F(NV) spmv_runs_t<double, NV>(nchunks, ntiles, chunks, toff, sg, (const double *)vt, (const double *)x, (double *)y, mode, (const double *)b, s)
+#define F(NV) spmv_runs_t<double, NV>(n, slots, nchunks, ntiles, chunks, toff, sg, (const double *)vt, (const double *)x, (double *)y, mode, (const double *)b, s)
         NV_DISPATCH(nv, F)
 #undef F
     } else {
-#define F(NV) spmv_runs_t<float, NV>(nchunks, ntiles, chunks, toff, sg, (const float *)vt, (const float *)x, (float *)y, mode, (const float *)b, s)
+#define F(NV) spmv_runs_t<float, NV>(n, slots, nchunks, ntiles, chunks, toff, sg, (const float *)vt, (const float *)x, (float *)y, mode, (const float *)b, s)
         NV_DISPATCH(nv, F)
 #undef F
     }

@@ -54,14 +54,14 @@ int get_spmv_run_rows();
 // offset}, both multiples of 4).  Tile t's segments (runs of at most 3
 // consecutive columns of each chunk's first row, c0 | len << 30) at
 // sg[toff[t].y + 4s + slot], its values at vt[(toff[t].x + 4e + slot) * 8 + q].
-// Same modes and the same results, bit for bit, as spmv().  FP64 nv 8, 16, 32
+// n rows, slots values.  Same modes and the same results, bit for bit, as spmv().  FP64 nv 8, 16, 32
 // and FP32 nv 16, 32.
 bool spmv_runs_supported(Prec p, int nv);
 // kernel form of the run product (per host thread): 0 = each segment's x rows
 // gathered into registers, 1 = copied into shared memory one segment ahead
 void set_spmv_run_form(int f);
 int get_spmv_run_form();
-void spmv_runs(Prec p, int nv, i64 nchunks, i64 ntiles, const int4 *chunks, const longlong2 *toff, const int *sg,
+void spmv_runs(Prec p, int nv, i64 n, i64 slots, i64 nchunks, i64 ntiles, const int4 *chunks, const longlong2 *toff, const int *sg,
                const void *vt, const void *x, void *y, int mode, const void *b, cudaStream_t s);
 
 // ---- Gauss-Seidel sweeps ----------------------------------------------------
