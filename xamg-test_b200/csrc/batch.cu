@@ -27,7 +27,7 @@ __device__ __forceinline__ int seg_of(const i64 *segoff, int nseg, i64 i) {
 // Stage 1 of the per-segment canonical inner products: chunks of 256 rows of
 // one segment (counted from the segment's first row), in the order and with the
 // split of the whole-vector dots (dots.cuh).  AL: the vectors lie on boundaries of
-// the loads (two elements); else element by element.
+// the loads (dot_ld); else element by element.
 template <class TI, int NV, int ND, bool SH, bool AL>
 __global__ void __launch_bounds__(256, ND == 1 ? 4 : 2) k_segdot1(int nseg, const i64 *__restrict__ segoff,
                                                  const i64 *__restrict__ cstart, i64 nch, int W,
@@ -35,7 +35,8 @@ __global__ void __launch_bounds__(256, ND == 1 ? 4 : 2) k_segdot1(int nseg, cons
                                                  const TI *__restrict__ a1, const TI *__restrict__ b1,
                                                  const TI *__restrict__ a2, const TI *__restrict__ b2,
                                                  double *__restrict__ part) {
-    constexpr int V = DotShape<NV>::V, C = ND * V;
+    typedef DotShape<TI, NV, ND> S;
+    constexpr int V = S::V, C = ND * V;
     __shared__ double sm[8 * C * 32];
     const int lane = threadIdx.x & 31;
     const i64 w = (i64)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), g = w / W;
@@ -50,9 +51,9 @@ __global__ void __launch_bounds__(256, ND == 1 ? 4 : 2) k_segdot1(int nseg, cons
         const i64 r0 = segoff[s] + (g - cstart[s]) * 256;
         dot_chunk<TI, NV, ND, SH, AL>(A, B, r0, (int)min((i64)256, segoff[s + 1] - r0), W, sub, v);
     }
-    if (!dot_join<NV>(W, sub, sm, v) || g >= nch) return;
-    dot_fold_lanes<NV>(v);
-    if (lane < DotShape<NV>::TPR)
+    if (!dot_join<S>(W, sub, sm, v) || g >= nch) return;
+    dot_fold_lanes<S>(v);
+    if (lane < S::TPR)
 #pragma unroll
         for (int d = 0; d < ND; ++d)
 #pragma unroll
@@ -178,18 +179,24 @@ static void segdots_t(int nseg, const i64 *segoff, const i64 *cstart, i64 nch, i
         const TI *A0 = (const TI *)a[0], *B0 = (const TI *)b[0];
         const TI *A1 = nd > 1 ? (const TI *)a[1] : A0, *B1 = nd > 1 ? (const TI *)b[1] : B0;
         const TI *A2 = nd > 2 ? (const TI *)a[2] : A0, *B2 = nd > 2 ? (const TI *)b[2] : B0;
-        const DotSplit sp = dot_split<NV>(nch, sm_count());
         const bool sh = nd == 3 && A1 == A0 && B1 == A0 && A2 == B0 && B2 == B0;
+        const i64 bytes = (sh ? 2 : 2 * nd) * nch * 256 * NV * (i64)sizeof(TI);
         uintptr_t low = 0;
         for (int d = 0; d < nd; ++d) low |= (uintptr_t)a[d] | (uintptr_t)b[d];
-        const bool al = low % (DotShape<NV>::V * sizeof(TI)) == 0;
 #define L(ND, SH, AL)                                                                               \
-    k_segdot1<TI, NV, ND, SH, AL><<<sp.blocks, 32 * sp.warps, 0, s>>>(nseg, segoff, cstart, nch, sp.W, A0, B0, A1, B1, A2, \
-                                                                      B2, part)
-#define LA(ND) { if (al) L(ND, false, true); else L(ND, false, false); }
+    {                                                                                               \
+        const DotSplit sp = dot_split<DotShape<TI, NV, ND>>(nch, sm_count(), bytes, 4);             \
+        k_segdot1<TI, NV, ND, SH, AL><<<sp.blocks, 32 * sp.warps, 0, s>>>(nseg, segoff, cstart, nch, sp.W, A0, B0, A1, \
+                                                                          B1, A2, B2, part);        \
+    }
+#define LA(ND)                                                                                      \
+    {                                                                                               \
+        if (low % std::min<size_t>(16, DotShape<TI, NV, ND>::V * sizeof(TI)) == 0) L(ND, false, true) \
+        else L(ND, false, false)                                                                    \
+    }
         if (nd == 1) LA(1)
         else if (nd == 2) LA(2)
-        else if (sh && al) L(3, true, true);
+        else if (sh && low % std::min<size_t>(16, DotShape<TI, NV, 3>::V * sizeof(TI)) == 0) L(3, true, true)
         else LA(3)
 #undef LA
 #undef L

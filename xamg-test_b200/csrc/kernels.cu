@@ -1192,9 +1192,15 @@ struct DotPairs {
     const TI *a[4];
     const TI *b[4];
 };
-template <class TI, int NV, int ND, bool SH>
-__global__ void __launch_bounds__(256, ND == 1 ? 4 : 2) k_dot1(i64 n, i64 nch, int W, DotPairs<TI> pr, double *__restrict__ part) {
-    constexpr int V = DotShape<NV>::V, C = ND * V;
+// threads of a block at most, and blocks of an SM at least
+template <class TI, int NV, int ND> struct DotBounds {
+    static constexpr int NT = DotShape<TI, NV, ND>::TPR == 1 ? 128 : 256;
+    static constexpr int MIN = (ND == 1 || (NV == 1 && sizeof(TI) == 4) ? 1024 : 512) / NT;
+};
+template <class TI, int NV, int ND, bool SH, bool AL>
+__global__ void __launch_bounds__(DotBounds<TI, NV, ND>::NT, DotBounds<TI, NV, ND>::MIN) k_dot1(i64 n, i64 nch, int W, DotPairs<TI> pr, double *__restrict__ part) {
+    typedef DotShape<TI, NV, ND> S;
+    constexpr int V = S::V, C = ND * V;
     __shared__ double sm[8 * C * 32];
     const int lane = threadIdx.x & 31;
     const i64 w = (i64)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), c = w / W;
@@ -1203,10 +1209,10 @@ __global__ void __launch_bounds__(256, ND == 1 ? 4 : 2) k_dot1(i64 n, i64 nch, i
 #pragma unroll
     for (int d = 0; d < ND; ++d) { A[d] = pr.a[d]; B[d] = pr.b[d]; }
     double v[C];
-    if (c < nch) dot_chunk<TI, NV, ND, SH>(A, B, c * 256, (int)min((i64)256, n - c * 256), W, sub, v);
-    if (!dot_join<NV>(W, sub, sm, v) || c >= nch) return;
-    dot_fold_lanes<NV>(v);
-    if (lane < DotShape<NV>::TPR)
+    if (c < nch) dot_chunk<TI, NV, ND, SH, AL>(A, B, c * 256, (int)min((i64)256, n - c * 256), W, sub, v);
+    if (!dot_join<S>(W, sub, sm, v) || c >= nch) return;
+    dot_fold_lanes<S>(v);
+    if (lane < S::TPR)
 #pragma unroll
         for (int d = 0; d < ND; ++d)
 #pragma unroll
@@ -1359,14 +1365,22 @@ static void dots_t(i64 n, int nd, const void *const *a, const void *const *b, do
         return;
     }
     note_launch(2);
-    const DotSplit sp = dot_split<NV>(nch, sm_count());
     const bool sh = nd == 3 && pr.a[1] == pr.a[0] && pr.b[1] == pr.a[0] && pr.a[2] == pr.b[0] && pr.b[2] == pr.b[0];
-#define L(ND, SH) k_dot1<TI, NV, ND, SH><<<sp.blocks, 32 * sp.warps, 0, s>>>(n, nch, sp.W, pr, part)
-    if (nd == 1) L(1, false);
-    else if (nd == 2) L(2, false);
-    else if (sh) L(3, true);
-    else if (nd == 3) L(3, false);
-    else L(4, false);
+    const i64 bytes = (sh ? 2 : 2 * nd) * n * NV * (i64)sizeof(TI);
+    // one pair of FP32 vectors is read 16 bytes a lane where both allow it
+    const bool al = (((uintptr_t)pr.a[0] | (uintptr_t)pr.b[0]) & 15) == 0;
+#define L(ND, SH, AL)                                                                               \
+    {                                                                                               \
+        const DotSplit sp = dot_split<DotShape<TI, NV, ND>>(nch, sm_count(), bytes, 4);             \
+        k_dot1<TI, NV, ND, SH, AL><<<sp.blocks, 32 * sp.warps, 0, s>>>(n, nch, sp.W, pr, part);     \
+    }
+    constexpr bool wide = sizeof(TI) == 4 && NV >= 4;
+    if (nd == 1 && wide && !al) L(1, false, !wide)
+    else if (nd == 1) L(1, false, true)
+    else if (nd == 2) L(2, false, true)
+    else if (sh) L(3, true, true)
+    else if (nd == 3) L(3, false, true)
+    else L(4, false, true)
 #undef L
     if (!reduce) {
         note_launch(-1);
@@ -1645,7 +1659,7 @@ __global__ void __launch_bounds__(256, 2) k_bicg_xr(i64 n, i64 nch, int W, const
                                                  T *__restrict__ x, const T *__restrict__ s,
                                                  const T *__restrict__ t, T *__restrict__ r,
                                                  const T *__restrict__ r0, double *__restrict__ part) {
-    typedef DotShape<NV> S;
+    typedef DotShape<T, NV, 2> S;
     constexpr int V = S::V, U = sizeof(T) * V <= 8 ? 4 : 2;
     __shared__ double sm[8 * V * 32];
     const int lane = threadIdx.x & 31, q = lane / S::TPR, k0 = lane % S::TPR * V, JW = S::TPR / W;
@@ -1698,8 +1712,8 @@ __global__ void __launch_bounds__(256, 2) k_bicg_xr(i64 n, i64 nch, int W, const
             }
             tree.push(i, acc);
         }
-    if (!dot_join<NV>(W, sub, sm, acc) || c >= nch) return;
-    dot_fold_lanes<NV>(acc);
+    if (!dot_join<S>(W, sub, sm, acc) || c >= nch) return;
+    dot_fold_lanes<S>(acc);
     if (lane < S::TPR)
 #pragma unroll
         for (int e = 0; e < V; ++e) part[(i64)(k0 + e) * nch + c] = acc[e];
@@ -2263,7 +2277,7 @@ static void bicg_groups_t(int grp, i64 n, const BicgScalars &sc, const void *a0,
             k_bicg_p<T, NV, 1><<<g, 256, 0, s>>>(tot, sc.c1, sc.beta, (const T *)a0, (const T *)a1, (T *)a2, (T *)a5);
     } else {
         const i64 nch = (n + 255) / 256;
-        const DotSplit sp = dot_split<NV>(nch, sm_count());
+        const DotSplit sp = dot_split<DotShape<T, NV, 2>>(nch, sm_count(), 0, 8);
         k_bicg_xr<T, NV><<<sp.blocks, 32 * sp.warps, 0, s>>>(
             n, nch, sp.W, sc.ac, sc.oc, sc.omega, (const T *)a0, (const T *)a1, (T *)a2, (const T *)a3, (const T *)a4,
             (T *)a5, (const T *)a6, part);
