@@ -165,12 +165,17 @@ void RunPlan::add_values(const HostCsr &h, Prec p) {
 // (us, runs / best CSR kernel: FP32 NV 16 27-point 32^3 7.5 / 6.5, 64^3 24 / 33,
 // 7-point 64^3 14.1 / 11.4, 100^3 55.7 / 58.8; FP64 NV 8 27-point 64^3 38.9 / 36.4,
 // with b - A x 49.8 / 38.1, 100^3 133 / 134 and 152 / 144, 128^3 239 / 272 and
-// 282 / 292, 7-point 100^3 76 / 71).  Coarse operators, of 43 to 160 entries a
-// row, have few rows in common runs: there the rows side by side are ahead at
-// every width (the products of a hierarchy's level, FP32 NV 32 63049 rows 77 / 37,
-// 250000 rows 92 / 69, NV 16 250000 rows 55 / 46).
+// 282 / 292, 7-point 100^3 76 / 71).  From 28 entries a row on, whatever part of
+// them lies in chunks of eight rows, a CTA's values no longer fit its stage (32 a
+// chunk) and the rows side by side are ahead at every width: 33-point (31 a row) 32^3
+// FP64 NV 8 19.4 / 7.9, NV 32 42.6 / 19.5, FP32 NV 32 12.8 / 12.5, 64^3 FP64 NV 16 131 / 84
+// (but FP32 NV 16 48.2 / 49.9, and 3 x 3 x 5 48^3 17.4 / 25.0); 3 x 3 x 5 (43) 64^3 FP64 NV 16
+// 153 / 92, FP32 NV 32 111 / 90;
+// 5 x 5 x 5 (118) 64^3, 89 % of the entries in full chunks, 509 / 241 and 340 / 236; the
+// first coarse level of the 27-point 100^3 (44, 96 %) 184 / 93 and 124 / 90.  At 24 a row
+// (5 x 5, 64^3) the runs are ahead, FP64 NV 16 55.0 / 68.4 (tile-staged 57.3).
 static bool runs_by_default(Prec p, int nv, i64 n, i64 nnz) {
-    if (nnz >= 32 * n) return false;
+    if (nnz >= 28 * n) return false;
     if (nv * (i64)prec_size(p) >= 128) return true;
     return nnz >= 16 * n && n > (p == Prec::F64 ? 1000000 : 65536);
 }

@@ -406,8 +406,7 @@ __global__ void __launch_bounds__(128) k_spmv_rows(i64 n, const int *__restrict_
 // SpMV variant selection: 0, 1, 2 = row kernel with gather batches of 4, 8,
 // 16 entries; 3, 4 = tile-staged kernel with batches of 4, 8; 5, 6 = the same
 // with a plain row loop unrolled 4, 8 times; 8 = rows side by side; 10 + k = streaming kernel
-// walking k tiles per CTA; -1 = default (6 when NV*sizeof(T) >= 64 bytes,
-// else 0).
+// walking k tiles per CTA; -1 = default (default_variant).
 static thread_local int g_spmv_variant = -1;
 void set_spmv_variant(int v) { g_spmv_variant = v; }
 static int g_run_rows = 8;
@@ -436,8 +435,9 @@ int sm_count() {
 //   rows of 16 entries and more, any width: the rows side by side (irregular
 //   4000 rows of 41, FP64 NV 4 8.3 / 13.5 / 16.2 / 17.8; FP32 NV 16 7.7 / 12.6 /
 //   12.8 / 16.9; 27-point 24^3 FP32 NV 8 3.9 / 4.7 / 4.9 / 6.0), but
-//   wide rows of less than 32, many of them: tile-staged (27-point 64^3 FP32 NV 16
-//   47 / 41 / 44 / 34; 24^3 4.1 / 4.8 / 5.1 / 5.0), and
+//   wide rows of less than 28, many of them: tile-staged (27-point 64^3 FP32 NV 16
+//   47 / 41 / 44 / 34; 24^3 4.1 / 4.8 / 5.1 / 5.0; of 31 side by side, 33-point 64^3 FP64
+//   NV 16 84 and tile-staged 100, NV 8 54 and 70), and
 //   FP64 NV 1, many rows: GB 8 (27-point 40^3 7.7 / 8.9 / 7.3 / 11.3, irregular
 //   55799 rows 24 / 27 / 21 / 32; 4000 rows 11.1 / 17.3 / 11.3 / 15.1);
 //   shorter rows: GB 4 (7-point 113x97x101 FP32 NV 8 60 / 33 / 43 / 45, FP64 NV 16
@@ -452,7 +452,7 @@ static int default_variant(i64 n, i64 nnz) {
     constexpr bool f64 = sizeof(T) == 8;
     if (nnz >= 16 * n) {
         if (f64 && NV == 1) return n <= 32768 ? 8 : 1;
-        return TPR <= 2 || nnz >= 32 * n || n <= 20000 ? 8 : 6;
+        return TPR <= 2 || nnz >= 28 * n || n <= 20000 ? 8 : 6;
     }
     if (TPR == 1) return f64 ? 1 : 0;
     return TPR >= 4 && nnz < 0 ? (n <= 8192 ? 8 : 6) : 0;
