@@ -1653,7 +1653,7 @@ struct Krylov : Solver {
     // GRID_ITERS of them.  Not while kernels are timed one by one.
     static constexpr int GRID_ITERS = 256;
     void setup_grid(i64 n) {
-        if (precond || reordered || cg || !xk::bicg_grid_fits(n)) return;
+        if (precond || reordered || cg || !xk::bicg_grid_fits(prec, nv, n, A->h.rp.data())) return;
         // one allocation: partials, residuals with {error flag, iterations run}
         // behind them, the second buffers of p and v
         const size_t vec = xk::bicg_grid_fly(prec, nv) ? (size_t)n * nv * prec_size(prec) : 0;

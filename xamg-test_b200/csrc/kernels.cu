@@ -1782,7 +1782,7 @@ __device__ __forceinline__ void bicg_epi_col(int k, const double *val, const Bic
 // Whole BiCGStab iterations (no preconditioner) in one cooperative launch.  On
 // small systems the iteration above is eight launches of 2 to 5 us with little in
 // them, the gaps between, and a host read; here a CTA keeps its chunks of 256
-// rows (their matrix rows in shared memory, where they fit) and the grid meets
+// rows (their matrix rows in shared memory) and the grid meets
 // only where a product needs all rows: at the three inner products, whose chunk
 // partials are also the barrier.  A partial is published in two 64-bit words of
 // 32 value bits and the iteration's number each, after a fence behind the CTA's
@@ -1919,10 +1919,9 @@ template <class T, int V> struct GridP {
     }
 };
 // entries j0 .. j1 - 1 of one row of a product, GB entries and their gathers at a
-// time; the matrix from shared memory (SM) or global
-template <class T, int NV, int GB, bool SM, class X>
-__device__ __forceinline__ void grid_row(const int *__restrict__ ci, const T *__restrict__ va, int j0, int j1, int k0,
-                                         const X &x, T (&acc)[Shape<T, NV>::V]) {
+// time; the matrix from shared memory
+template <class T, int NV, int GB, class X>
+__device__ __forceinline__ void grid_row(const int *ci, const T *va, int j0, int j1, int k0, const X &x, T (&acc)[Shape<T, NV>::V]) {
     constexpr int V = Shape<T, NV>::V;
 #pragma unroll
     for (int e = 0; e < V; ++e) acc[e] = T(0);
@@ -1932,8 +1931,8 @@ __device__ __forceinline__ void grid_row(const int *__restrict__ ci, const T *__
 #pragma unroll
         for (int k = 0; k < GB; ++k) {
             const int u = min(j + k, j1 - 1);  // past the end: the last entry again, not added
-            c[k] = SM ? ci[u] : __ldg(ci + u);
-            v[k] = SM ? va[u] : __ldg(va + u);
+            c[k] = ci[u];
+            v[k] = va[u];
         }
 #pragma unroll
         for (int k = 0; k < GB; ++k) x.get((i64)c[k] * NV + k0, xv[k]);
@@ -1951,7 +1950,7 @@ __global__ void __launch_bounds__(BicgGridShape<T, NV>::NT, BicgGridShape<T, NV>
     constexpr int GB = V * (FLY ? 3 : 1) * (int)sizeof(T) > 24 ? 4 : 8;
     extern __shared__ __align__(16) unsigned char raw[];
     T *sa = reinterpret_cast<T *>(raw), *sb = sa + NV * PK;
-    // the CTA's rows of the matrix, when they fit
+    // the CTA's rows of the matrix
     T *sm_v = sb + NV * PK;
     int *sm_c = reinterpret_cast<int *>(sm_v + ecap), *sm_r = sm_c + ecap;
     __shared__ double val[3 * NV], rho[NV], alpha[NV], omega[NV], beta[NV], c1[NV], ac[NV], oc[NV], iconv[NV],
@@ -1969,13 +1968,15 @@ __global__ void __launch_bounds__(BicgGridShape<T, NV>::NT, BicgGridShape<T, NV>
     const int clo = blockIdx.x * cpc, chi = min(clo + cpc, nch);  // its chunks
     const i64 lo = (i64)clo * 256, hi = (i64)chi * 256 < n ? (i64)chi * 256 : n;
     const int e0 = __ldg(g.rp + lo), e1 = __ldg(g.rp + hi);
-    const bool kept = e1 - e0 <= ecap;
+    if (e1 - e0 > ecap) {  // not a system that bicg_grid_fits
+        if (tid == 0) atomicExch(g.err, 2);
+        return;
+    }
     for (int q = tid; q <= (int)(hi - lo); q += NT) sm_r[q] = __ldg(g.rp + lo + q);
-    if (kept)
-        for (int j = tid; j < e1 - e0; j += NT) {
-            sm_v[j] = __ldg(g.va + e0 + j);
-            sm_c[j] = __ldg(g.ci + e0 + j);
-        }
+    for (int j = tid; j < e1 - e0; j += NT) {
+        sm_v[j] = __ldg(g.va + e0 + j);
+        sm_c[j] = __ldg(g.ci + e0 + j);
+    }
     __syncthreads();
 
     // partials of this chunk's pairs (operands in sa, sb), one warp per pair and
@@ -2030,12 +2031,8 @@ __global__ void __launch_bounds__(BicgGridShape<T, NV>::NT, BicgGridShape<T, NV>
         __syncthreads();
         return bad == 0;
     };
-#define GROW(...)                                                                                  \
-    {                                                                                              \
-        const int j0 = sm_r[row - lo], j1 = sm_r[row - lo + 1];                                    \
-        if (kept) grid_row<T, NV, GB, true>(sm_c, sm_v, j0 - e0, j1 - e0, k0, __VA_ARGS__, acc); \
-        else grid_row<T, NV, GB, false>(g.ci, g.va, j0, j1, k0, __VA_ARGS__, acc);                 \
-    }
+#define GROW(...)                                                                                              \
+    grid_row<T, NV, GB>(sm_c, sm_v, sm_r[row - lo] - e0, sm_r[row - lo + 1] - e0, k0, __VA_ARGS__, acc)
     int it = it0;
     for (; it < it1; ++it) {
         T *const pn = g.p[FLY ? it & 1 : 0], *const vn = g.v[FLY ? it & 1 : 0];
@@ -2208,26 +2205,38 @@ size_t bicg_grid_bytes(i64 n, int nv) {
     return sizeof(BicgGridSlot) * (size_t)(5 * nv * nch + nch);
 }
 
+// The launch of a system of n rows: chunks per CTA (two CTAs of 256 threads on an
+// SM when there are chunks for them), entries of the matrix that a CTA can hold.
+struct BicgGridPlan {
+    int nch, cpc, ecap;
+    size_t smem;
+    int grid() const { return (nch + cpc - 1) / cpc; }
+};
+template <class T, int NV> static BicgGridPlan bicg_grid_plan(i64 n) {
+    BicgGridPlan p;
+    p.nch = (int)((n + 255) / 256);
+    const int per = BicgGridShape<T, NV>::NT == 256 && p.nch > sm_count() ? 2 : 1, slots = per * sm_count();
+    p.cpc = (p.nch + slots - 1) / slots;
+    const size_t room = (size_t)(per == 1 ? 220 : 110) * 1024, base = BicgGridShape<T, NV>::SMEM;
+    const size_t rows = sizeof(int) * ((size_t)p.cpc * 256 + 1);
+    p.ecap = room > base + rows ? (int)((room - base - rows) / (sizeof(T) + 4)) / 2 * 2 : 0;
+    p.smem = base + rows + (size_t)p.ecap * (sizeof(T) + 4);
+    return p;
+}
+
 template <class T, int NV, bool FLY>
 static cudaError_t bicg_grid_l(const BicgGridArgs &a, i64 n, int it0, int it1, const BicgScalars &sc, cudaStream_t s) {
     auto k = k_bicg_grid<T, NV, FLY>;
-    constexpr int NT = BicgGridShape<T, NV>::NT;
-    // two CTAs of 256 threads on an SM when there are chunks for them
-    int nch = (int)((n + 255) / 256);
-    const int per = NT == 256 && nch > sm_count() ? 2 : 1, slots = per * sm_count();
-    int cpc = (nch + slots - 1) / slots;
-    const size_t room = (size_t)(per == 1 ? 220 : 110) * 1024, base = BicgGridShape<T, NV>::SMEM;
-    const size_t rows = sizeof(int) * ((size_t)cpc * 256 + 1);
-    int ecap = room > base + rows ? (int)((room - base - rows) / (sizeof(T) + 4)) / 2 * 2 : 0;
-    const size_t smem = base + rows + (size_t)ecap * (sizeof(T) + 4);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    BicgGridPlan p = bicg_grid_plan<T, NV>(n);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
     if (e != cudaSuccess) return e;
     BicgGrid<T> g{a.rp, a.ci, (const T *)a.va, (const T *)a.r0, (T *)a.r, (T *)a.x, (T *)a.s, (T *)a.t,
                   {(T *)a.p[0], (T *)a.p[1]}, {(T *)a.v[0], (T *)a.v[1]}, (BicgGridSlot *)a.slots, a.hist, a.err, a.done};
     BicgScalars scv = sc;
-    void *args[] = {&g, &n, &nch, &cpc, &ecap, &it0, &it1, &scv};
+    void *args[] = {&g, &n, &p.nch, &p.cpc, &p.ecap, &it0, &it1, &scv};
     note_launch();
-    return cudaLaunchCooperativeKernel((const void *)k, dim3((unsigned)((nch + cpc - 1) / cpc)), dim3(NT), args, smem, s);
+    return cudaLaunchCooperativeKernel((const void *)k, dim3((unsigned)p.grid()), dim3(BicgGridShape<T, NV>::NT), args,
+                                       p.smem, s);
 }
 
 // Gathering two or three vectors for each entry against one more meeting: up to
@@ -2237,11 +2246,33 @@ static cudaError_t bicg_grid_l(const BicgGridArgs &a, i64 n, int it0, int it1, c
 template <class T, int NV> constexpr bool bicg_fly_v = NV * sizeof(T) <= 32;
 bool bicg_grid_fly(Prec p, int nv) { return nv * (p == Prec::F64 ? 8 : 4) <= 32; }
 
-// Two chunks per SM: at 40^3 (250 chunks) every operator and width gains (7-point
-// NV 1 57.9 -> 19.1 us per iteration, 27-point NV 16 247 -> 101), at 64^3 the
-// separate kernels have work enough (7-point NV 1 62 -> 53, NV 8 157 -> 139, but
-// 27-point NV 1 133 -> 271, its matrix no longer in shared memory).
-bool bicg_grid_fits(i64 n) { return n > 0 && (n + 255) / 256 <= 2 * sm_count(); }
+// Two chunks per SM, and every CTA's rows of the matrix in shared memory: then the
+// launch is ahead (us per iteration, separate kernels / this, FP64: 7-point 40^3 NV 1
+// 51 / 19, NV 16 70 / 63; 27-point 40^3 NV 8 70 / 59; 3 x 3 x 5 32^3 NV 16 77 / 59), and
+// without them behind (27-point 40^3 NV 16 80 / 98; 3 x 3 x 5 40^3 NV 1 71 / 110; 5 x 5 x 5
+// 16^3 NV 4 61 / 119, 42^3 NV 1 120 / 509), also beyond two chunks (27-point 64^3 NV 1
+// 133 / 271).  rp: the row pointers on the host.
+template <class T, int NV> static bool grid_fits_t(i64 n, const int *rp) {
+    const BicgGridPlan p = bicg_grid_plan<T, NV>(n);
+    if (p.nch > 2 * sm_count()) return false;
+    for (int c = 0; c < p.nch; c += p.cpc)
+        if (rp[std::min<i64>(n, (i64)(c + p.cpc) * 256)] - rp[(i64)c * 256] > p.ecap) return false;
+    return true;
+}
+bool bicg_grid_fits(Prec p, int nv, i64 n, const int *rp) {
+    if (n <= 0) return false;
+    bool ok = false;
+    if (p == Prec::F64) {
+#define F(NV) ok = grid_fits_t<double, NV>(n, rp)
+        NV_DISPATCH(nv, F)
+#undef F
+    } else {
+#define F(NV) ok = grid_fits_t<float, NV>(n, rp)
+        NV_DISPATCH(nv, F)
+#undef F
+    }
+    return ok;
+}
 
 cudaError_t bicg_grid(Prec p, int nv, const BicgGridArgs &a, i64 n, int it0, int it1, const BicgScalars &sc,
                       cudaStream_t s) {

@@ -216,7 +216,7 @@ struct BicgGridArgs {
     double *hist;
     int *err, *done;
 };
-bool bicg_grid_fits(i64 n);
+bool bicg_grid_fits(Prec p, int nv, i64 n, const int *rp_host);
 bool bicg_grid_fly(Prec p, int nv);
 size_t bicg_grid_bytes(i64 n, int nv);
 cudaError_t bicg_grid(Prec p, int nv, const BicgGridArgs &a, i64 n, int it0, int it1, const BicgScalars &sc,
