@@ -102,6 +102,7 @@ Context &ctx();
 // recorded by their form: single-process order (GS_GRID), hybrid blocks with
 // one CTA per block and the x tile in shared memory or x through the L1
 // (GS_TILE, GS_WINDOW), one warp per block (GSW_*); GS covers the other paths.
+// GS_GATHER keeps its number and is not recorded.
 enum class KClass : int {
     GS = 0, SPMV = 1, GS_GRID = 2, GS_TILE = 3, GS_WINDOW = 4, GS_GATHER = 5,
     GSW_TILE = 6, GSW_WINDOW = 7, GSW_GATHER = 8

@@ -278,13 +278,7 @@ void GsPlan::build(const HostCsr &A, i64 brows_, GsMode mode_) {
     XCUDA(cudaMemset(sync.p, 0, kSyncBytes));
 }
 
-// Level-ordered matrix copy of one sweep direction.  Rows are stored in
-// schedule order ((block,) level, row); every level group is padded with
-// empty rows (row id -1) to a multiple of 4 rows and every row's in-block
-// entries (CSR order) are padded with column -1 to a multiple of 4, so all row
-// and entry ranges handed to one CTA start on 16-byte boundaries and span
-// multiples of 16 bytes (the TMA bulk-copy rule).  One descriptor {r0, r1, e0,
-// e1} per (level, CTA) tells each CTA what to stage.
+// The entries of A outside each row's block, in CSR order (see GsPlan::aoff).
 void GsPlan::build_offblock(const HostCsr &A, Prec p) {
     if (brows == 0) return;
     HostCsr off;
@@ -316,7 +310,6 @@ void GsPlan::build_offblock(const HostCsr &A, Prec p) {
 // kMaxSlots slots at once.
 constexpr int kSlotAhead = xk::kGsSlotAhead;
 constexpr int kMaxSlots = 4096;
-
 
 void GsPlan::build_slots(int d, const std::vector<int> &order, const std::vector<int> &groups,
                          const std::vector<int> &blev, const std::vector<int> &lrp, const std::vector<int> &lci) {
@@ -480,8 +473,6 @@ bool GsPlan::build_items(int d, int rows, const HostCsr &A, Prec p, const std::v
     L.rows = rows;
     L.ientries = 0;
     std::vector<std::pair<int, int>> lr;  // (-groups, row) of one level
-    std::vector<int> col;
-    std::vector<double> val;
     for (int b = 0; b < nb; ++b) {
         std::vector<int> lastitem;  // last item and items of every level
         std::vector<int> cnt;
