@@ -420,9 +420,9 @@ GS_FORM_KERNEL = {"gs_grid": "k_gs_flow<float,16> (one sweep on the whole device
                   "gsw_tile": "k_gsw<float,16,1> (hybrid blocks, one warp each, x tile)",
                   "gsw_window": "k_gsw<float,16,2> (hybrid blocks, one warp each, slot window)",
                   "gsw_gather": "k_gsw<float,16,0> (hybrid blocks, one warp each, per-level gather)"}
-# DRAM bytes (read + write) per algorithmic byte of a sweep form, from an ncu
-# capture of the form that runs (none taken of the current kernels yet)
-GS_TRAFFIC_RATIO = {}
+# DRAM bytes (read + write) per algorithmic byte of a sweep form, from the ncu
+# capture in profiles/kernels_of_the_listed_cases.md
+GS_TRAFFIC_RATIO = {"gs_window": 0.987}
 
 
 def gs_roofline(rec, solve_ms, rows):

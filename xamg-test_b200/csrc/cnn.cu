@@ -229,10 +229,11 @@ __global__ void __launch_bounds__(128) k_conv3d(const bf16 *__restrict__ in, int
 // in shared memory for all boxes when they fit (WRES), else each chunk brings its
 // own.  Voxels outside the volume are zeros; outputs outside it are not stored.
 // Same sums as k_conv3d, chunk by chunk (the order of the kernel before).
-// Bound: mma.sync (half of its 550 TFLOP/s) and the shared-memory reads beside it,
-// four A and BN / 16 B fragments for BN / 2 mma.  48 -> 16 channels, 8 x 64^3: 283
-// us, 310 TFLOP/s; 605 us by the kernel before, which staged halo and weights for
-// 128 voxels at a time with nothing under way meanwhile.
+// Bound: the fragments' reads from shared memory (66 % of its wavefronts), four A
+// and BN / 16 B fragments for BN / 2 mma, and the tensor pipe behind them (60 % of its
+// cycles).  48 -> 16 channels, 8 x 64^3: 274 us, 318 TFLOP/s; 602 us by the kernel
+// before, which staged halo and weights for 128 voxels at a time with nothing under
+// way meanwhile.
 template <int BN, int BZ> struct BoxShape {
     static constexpr int NT = 32 * BZ, ROWS = (BZ + 2) * 100, HBYTES = 2 * ROWS * 16, WBYTES = 27 * BN * 32;
 };
@@ -445,7 +446,7 @@ __global__ void __launch_bounds__(32 * BZ, BN == 16 ? 16 / BZ : BZ == 8 || BN ==
 // a fragment of the gradient serves 3 or 4 taps, and every partial sum stays in
 // registers until the CTA's boxes are done (FP32 atomics, one per CTA and
 // weight).  Voxels outside the volume are zeros on both sides.
-// Bound: mma.sync (54 % of its cycles) and the fragments' latency.  cin 96, cout
+// Bound: the tensor pipe by mma.sync (53 % of its cycles) and the fragments' latency.  cin 96, cout
 // 32, 4 x 32^3: 90 us, 240 TFLOP/s; 569 us by the kernel before, which staged the
 // gradient and a shifted input once per tap and chunk.
 constexpr int WG_HALO = 4 * 10 * 10, WG_VOX = 128;

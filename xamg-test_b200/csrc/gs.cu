@@ -17,7 +17,8 @@
 //                barrier between two levels.
 //
 // What bounds them is the chain from level to level: the arrival of the
-// previous level's values, the rest of the row's FMA chain, the store.  Measured
+// previous level's values, the rest of the row's FMA chain, the store (k_gs_block
+// on 80^3 in 444 blocks: DRAM at 12 % of its rate, L1 39 %, issue 31 %).  Measured
 // (B200, both sweeps of one call, 27-point operators; before: one CTA barrier,
 // TMA wait and gather per level):
 //   k_gs_block FP32 NV=16, 444 blocks   64^3 227 -> 113 us, 80^3 367 -> 244 us

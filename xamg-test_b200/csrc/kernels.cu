@@ -312,7 +312,8 @@ __global__ void __launch_bounds__(256, LOOP == 1 ? 6 : 1) k_spmv_tile(i64 n, con
 // global memory, every column and value would take an L1 wavefront of its own
 // beside the gather's; staged tile by tile, rows wait for the longest of theirs
 // chunk after chunk.  Same per-row summation order as k_spmv.
-// Bound: L1 wavefronts of the gathers; on small operators the latency of a
+// Bound: the gathers, by the L1 (68 % of its rate on 55799 irregular rows, FP32 NV
+// 8) and their latency; on small operators the latency of a
 // step (irregular 4000 rows of 41 entries, FP32 NV 16: 7.7 us, tile-staged 16.9).
 // Eight entries a step where 16 cost registers or shared memory (FP64 NV 8, the
 // same operator: 9.1 us against 14.1).
